@@ -28,31 +28,53 @@ constexpr int BT = 128;
 constexpr int BWD_THREADS = 320;  // 8 softmax warps (two per TMEM lane quadrant), TMA warp, MMA warp
 constexpr float LOG2E_B = 1.4426950408889634f;
 
-// one warp per (b, t, h) row of D elements
-__global__ void attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
-                                  const float* __restrict__ lse, const float* __restrict__ sinks,
-                                  float* __restrict__ delta, float* __restrict__ dsinks,
-                                  int B, int T, int H, int D) {
-  const long rows = (long)B * T * H;
-  const int lane = threadIdx.x & 31;
-  for (long row = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); row < rows;
-       row += (long)gridDim.x * (blockDim.x >> 5)) {
+// delta[b, h, t] = sum_d O·dO, and the sinks' gradient. A stream of 4·D bytes per row: a block
+// takes 32 tokens x 8 heads, D / 8 lanes per row with one 16-byte load of each operand, and turns
+// the sums in shared memory so that they leave as whole 128-byte lines along t. The sink gradient
+// is one atomic per (32 tokens, head): with one per row, all rows of a head queued on one address
+// (2 x 4096 x 64 heads of 64: 379 us, now 35; without sinks, 2 x 4096 x 32 heads of 128: 59 us, now 31).
+constexpr int DELTA_T = 32, DELTA_H = 8;
+template <int D>
+__global__ void __launch_bounds__(256)
+attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
+                  const float* __restrict__ lse, const float* __restrict__ sinks,
+                  float* __restrict__ delta, float* __restrict__ dsinks, int T, int H) {
+  constexpr int LPR = D / 8;            // lanes per row
+  constexpr int PER = 256 / LPR;        // rows the block works on at once
+  __shared__ float sums[DELTA_H][DELTA_T + 1];
+  const int t0 = blockIdx.x * DELTA_T, h0 = blockIdx.y * DELTA_H, b = blockIdx.z;
+  const int li = threadIdx.x % LPR, first = threadIdx.x / LPR;
+#pragma unroll 4
+  for (int i = first; i < DELTA_T * DELTA_H; i += PER) {
+    const int t = t0 + i / DELTA_H, h = h0 + i % DELTA_H;
     float acc = 0.f;
-    for (int i = lane * 2; i < D; i += 64) {
-      const float2 a = unpack_bf16(*reinterpret_cast<const uint32_t*>(o + row * D + i));
-      const float2 g = unpack_bf16(*reinterpret_cast<const uint32_t*>(d_o + row * D + i));
-      acc += a.x * g.x + a.y * g.y;
+    if (t < T && h < H) {
+      const size_t at = (((size_t)b * T + t) * H + h) * D + li * 8;
+      const uint4 x = *reinterpret_cast<const uint4*>(o + at), y = *reinterpret_cast<const uint4*>(d_o + at);
+      const uint32_t* xu = &x.x; const uint32_t* yu = &y.x;
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 p = unpack_bf16(xu[j]), g = unpack_bf16(yu[j]);
+        acc += p.x * g.x + p.y * g.y;
+      }
     }
-    acc = warp_sum(acc);
-    if (lane == 0) {
-      const int h = (int)(row % H);
-      const long bt = row / H;
-      const int t = (int)(bt % T);
-      const int b = (int)(bt / T);
-      const size_t idx = ((size_t)b * H + h) * T + t;
-      delta[idx] = acc;
-      if (sinks && dsinks) atomicAdd(&dsinks[h], -__expf(sinks[h] - lse[idx]) * acc);
-    }
+#pragma unroll
+    for (int s = LPR / 2; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+    if (li == 0) sums[i % DELTA_H][i / DELTA_H] = acc;
+  }
+  __syncthreads();
+  const int t = t0 + (threadIdx.x & 31), h = h0 + (threadIdx.x >> 5);   // a warp per head
+  if (h >= H) return;
+  float ds = 0.f;
+  if (t < T) {
+    const size_t idx = ((size_t)b * H + h) * T + t;
+    const float acc = sums[threadIdx.x >> 5][threadIdx.x & 31];
+    delta[idx] = acc;
+    if (sinks && dsinks) ds = -__expf(sinks[h] - lse[idx]) * acc;
+  }
+  if (sinks && dsinks) {
+    ds = warp_sum(ds);
+    if ((threadIdx.x & 31) == 0) atomicAdd(&dsinks[h], ds);
   }
 }
 
@@ -495,10 +517,9 @@ static const char* attn_bwd_launch_d(const AttnArgs& a, cudaStream_t stream) {
   static bool configured[64] = {};
   if (!allow_dynamic_smem(kern, Cfg::SMEM_BYTES, configured))
     return "cudaFuncSetAttribute(max dynamic shared memory) failed";
-  const long rows = (long)a.B * a.T * a.H;
-  attn_delta_kernel<<<(int)min((rows + 7) / 8, 148L * 16), 256, 0, stream>>>(
+  attn_delta_kernel<D><<<dim3((a.T + DELTA_T - 1) / DELTA_T, (a.H + DELTA_H - 1) / DELTA_H, a.B), 256, 0, stream>>>(
       reinterpret_cast<const __nv_bfloat16*>(a.o), reinterpret_cast<const __nv_bfloat16*>(a.d_o), a.lse,
-      a.sinks, a.delta, a.dsinks, a.B, a.T, a.H, D);
+      a.sinks, a.delta, a.dsinks, a.T, a.H);
   dim3 grid((a.S + BT - 1) / BT, a.G, a.B);
   kern<<<grid, BWD_THREADS, Cfg::SMEM_BYTES, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? nullptr : "attention backward launch failed";

@@ -281,7 +281,9 @@ void attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o
   check_cuda(q, "q"); check_cuda(d_o, "do");
   c10::cuda::CUDAGuard guard(q.device());
   bux::AttnArgs a;
-  a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr(); a.o = o.data_ptr(); a.lse = lse.data_ptr<float>();
+  // O is read in 16-byte pieces; a view that starts between them (dO's start the tensor map checks) is copied
+  const Tensor o16 = reinterpret_cast<uintptr_t>(o.data_ptr()) % 16 == 0 ? o : o.clone();
+  a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr(); a.o = o16.data_ptr(); a.lse = lse.data_ptr<float>();
   a.d_o = d_o.data_ptr(); a.dq = dq.data_ptr(); a.dk = dk.data_ptr(); a.dv = dv.data_ptr(); a.delta = delta.data_ptr<float>();
   a.sinks = opt_f32(sinks);
   a.dsinks = dsinks.has_value() ? dsinks->data_ptr<float>() : nullptr;

@@ -269,6 +269,28 @@ def test_attention_bwd(cuda, d, h, g, t, window, sinks):
         assert rel_err(dsk, sk.grad) < 3e-2
 
 
+@pytest.mark.parametrize("d,h,g,t", [(64, 12, 4, 33), (128, 3, 1, 31), (64, 8, 8, 1), (128, 9, 3, 64)])
+def test_attention_sink_gradient_at_the_edges_of_its_tiles(cuda, d, h, g, t):
+    """32 tokens x 8 heads go together in the kernel that forms delta and the sinks' gradient.
+    Bound: every term of d sink is a bf16 product, off by 2^-8, and the terms partly cancel."""
+    from bux_b200.ops import kernels as K
+
+    torch.manual_seed(19)
+    q, do = (torch.randn(2, t, h, d, device=cuda).bfloat16() for _ in range(2))
+    k, v = (torch.randn(2, t, g, d, device=cuda).bfloat16() for _ in range(2))
+    sk = torch.randn(h, device=cuda).requires_grad_()
+    q.requires_grad_()
+    want, _ = ref.attention(q, k, v, causal=True, sinks=sk)
+    want.backward(do)
+    with torch.no_grad():
+        o, lse = K.attn_fwd(q, k, v, sinks=sk)
+        at = torch.empty(o.numel() + 1, device=cuda, dtype=o.dtype)[1:].view_as(o).copy_(o)  # starts between 16-byte pieces
+        for out in (o, at):
+            dq, _, _, dsk = K.attn_bwd(q, k, v, out, do, lse, sinks=sk)
+            assert rel_err(dsk, sk.grad) < 3e-2
+            assert t == 1 or rel_err(dq, q.grad) < 3e-2
+
+
 def _documents(t: int, lens, device):
     """Document ids [1, t] of a row packed with documents of the given lengths."""
     assert sum(lens) == t
