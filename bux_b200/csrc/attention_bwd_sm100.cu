@@ -38,7 +38,7 @@ template <int D>
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
                   const float* __restrict__ lse, const float* __restrict__ sinks,
-                  float* __restrict__ delta, float* __restrict__ dsinks, int T, int H) {
+                  float* __restrict__ delta, float* __restrict__ dsinks, int T, int H, bool o16) {
   constexpr int LPR = D / 8;            // lanes per row
   constexpr int PER = 256 / LPR;        // rows the block works on at once
   __shared__ float sums[DELTA_H][DELTA_T + 1];
@@ -50,7 +50,15 @@ attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __re
     float acc = 0.f;
     if (t < T && h < H) {
       const size_t at = (((size_t)b * T + t) * H + h) * D + li * 8;
-      const uint4 x = *reinterpret_cast<const uint4*>(o + at), y = *reinterpret_cast<const uint4*>(d_o + at);
+      const uint4 y = *reinterpret_cast<const uint4*>(d_o + at);
+      uint4 x;
+      if (o16) {
+        x = *reinterpret_cast<const uint4*>(o + at);
+      } else {   // O starts between 16-byte boundaries (dO's start the tensor map checks)
+        const unsigned short* p = reinterpret_cast<const unsigned short*>(o + at);
+        x = make_uint4(p[0] | (uint32_t)p[1] << 16, p[2] | (uint32_t)p[3] << 16, p[4] | (uint32_t)p[5] << 16,
+                       p[6] | (uint32_t)p[7] << 16);
+      }
       const uint32_t* xu = &x.x; const uint32_t* yu = &y.x;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -519,7 +527,7 @@ static const char* attn_bwd_launch_d(const AttnArgs& a, cudaStream_t stream) {
     return "cudaFuncSetAttribute(max dynamic shared memory) failed";
   attn_delta_kernel<D><<<dim3((a.T + DELTA_T - 1) / DELTA_T, (a.H + DELTA_H - 1) / DELTA_H, a.B), 256, 0, stream>>>(
       reinterpret_cast<const __nv_bfloat16*>(a.o), reinterpret_cast<const __nv_bfloat16*>(a.d_o), a.lse,
-      a.sinks, a.delta, a.dsinks, a.T, a.H);
+      a.sinks, a.delta, a.dsinks, a.T, a.H, reinterpret_cast<uintptr_t>(a.o) % 16 == 0);
   dim3 grid((a.S + BT - 1) / BT, a.G, a.B);
   kern<<<grid, BWD_THREADS, Cfg::SMEM_BYTES, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? nullptr : "attention backward launch failed";

@@ -96,7 +96,14 @@ void rmsnorm_bwd(const Tensor& x, const c10::optional<Tensor>& w, const Tensor& 
   const int d = (int)x.size(-1);
   c10::cuda::CUDAGuard guard(x.device());
   float* dwp = dw.has_value() ? dw->data_ptr<float>() : nullptr;
-  bux::rmsnorm_bwd(x.data_ptr(), opt_f32(w), dy.data_ptr(), rstd.data_ptr<float>(), dx.data_ptr(), dwp, x.numel() / d, d, stream_of(x));
+  Tensor part;
+  if (dwp) {
+    const int n = bux::rmsnorm_bwd_partials(x.numel() / d, d);
+    if (n > 0) part = at::empty({n, d}, dw->options());
+    else dw->zero_();
+  }
+  bux::rmsnorm_bwd(x.data_ptr(), opt_f32(w), dy.data_ptr(), rstd.data_ptr<float>(), dx.data_ptr(), dwp,
+                   part.defined() ? part.data_ptr<float>() : nullptr, x.numel() / d, d, stream_of(x));
 }
 // x viewed as [tokens, heads, D] with token stride stride_x (elements); y likewise.
 void norm_rope(bool bwd, const Tensor& x, const c10::optional<Tensor>& w, const Tensor& cos, const Tensor& sin,
@@ -281,9 +288,7 @@ void attn_bwd(const Tensor& q, const Tensor& k, const Tensor& v, const Tensor& o
   check_cuda(q, "q"); check_cuda(d_o, "do");
   c10::cuda::CUDAGuard guard(q.device());
   bux::AttnArgs a;
-  // O is read in 16-byte pieces; a view that starts between them (dO's start the tensor map checks) is copied
-  const Tensor o16 = reinterpret_cast<uintptr_t>(o.data_ptr()) % 16 == 0 ? o : o.clone();
-  a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr(); a.o = o16.data_ptr(); a.lse = lse.data_ptr<float>();
+  a.q = q.data_ptr(); a.k = k.data_ptr(); a.v = v.data_ptr(); a.o = o.data_ptr(); a.lse = lse.data_ptr<float>();
   a.d_o = d_o.data_ptr(); a.dq = dq.data_ptr(); a.dk = dk.data_ptr(); a.dv = dv.data_ptr(); a.delta = delta.data_ptr<float>();
   a.sinks = opt_f32(sinks);
   a.dsinks = dsinks.has_value() ? dsinks->data_ptr<float>() : nullptr;

@@ -15,45 +15,221 @@
 namespace bux {
 
 // ---------------------------------------------------------------- RMSNorm
-// One warp per row. x, y: [rows, d] bf16; w: [d] fp32 or null; rstd: [rows] fp32 out.
-template <int VEC>
-__global__ void rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w,
-                                   __nv_bfloat16* __restrict__ y, float* __restrict__ rstd,
-                                   int rows, int d, float eps) {
-  const int warps_per_block = blockDim.x >> 5;
-  const int row = blockIdx.x * warps_per_block + (threadIdx.x >> 5);
+__device__ __forceinline__ void unpack8(const uint4& v, float (&f)[8]) {
+  const uint32_t* u = &v.x;
+#pragma unroll
+  for (int j = 0; j < 4; ++j) { const float2 t = unpack_bf16(u[j]); f[2 * j] = t.x; f[2 * j + 1] = t.y; }
+}
+__device__ __forceinline__ uint4 pack8(const float (&f)[8]) {
+  return make_uint4(pack_bf16(f[0], f[1]), pack_bf16(f[2], f[3]), pack_bf16(f[4], f[5]), pack_bf16(f[6], f[7]));
+}
+// Eight fp32 gains from column 8 i (1 without gains); `w16`: w starts on a 16-byte boundary.
+__device__ __forceinline__ void load_gain8(const float* __restrict__ w, bool w16, int i, float (&g)[8]) {
+  if (w == nullptr) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) g[j] = 1.f;
+  } else if (w16) {
+    const float4 lo = reinterpret_cast<const float4*>(w)[2 * i], hi = reinterpret_cast<const float4*>(w)[2 * i + 1];
+    g[0] = lo.x; g[1] = lo.y; g[2] = lo.z; g[3] = lo.w; g[4] = hi.x; g[5] = hi.y; g[6] = hi.z; g[7] = hi.w;
+  } else {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) g[j] = w[i * 8 + j];
+  }
+}
+
+// One warp per row. x, y: [rows, d] bf16; w: [d] fp32 or null; rstd: [rows] fp32 out. NV > 0: the
+// row stays in registers, NV 16-byte loads per lane all in flight (rows up to 32 * 8 * NV wide); it
+// is a stream, bound by the bytes it keeps in flight: 16384 x 2048 took 49 us with the row read
+// a second time and one load in flight at a time, 31 now. NV = 0: rows of any width, read twice.
+template <int NV>
+__global__ void __launch_bounds__(256, NV > 0 ? 3 : 2)
+rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w, bool w16,
+                   __nv_bfloat16* __restrict__ y, float* __restrict__ rstd, int rows, int d, float eps) {
+  const int row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
   const int lane = threadIdx.x & 31;
   if (row >= rows) return;
   const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * d);
+  uint4* yr = reinterpret_cast<uint4*>(y + (size_t)row * d);
   const int nvec = d / 8;
+  constexpr int HELD = NV > 0 ? NV : 1;
+  uint4 held[HELD];
   float ss = 0.f;
-  for (int i = lane; i < nvec; i += 32) {
-    uint4 v = xr[i];
-    float2 a = unpack_bf16(v.x), b = unpack_bf16(v.y), c = unpack_bf16(v.z), e = unpack_bf16(v.w);
-    ss += a.x * a.x + a.y * a.y + b.x * b.x + b.y * b.y + c.x * c.x + c.y * c.y + e.x * e.x + e.y * e.y;
+  if (NV > 0) {
+#pragma unroll
+    for (int k = 0; k < HELD; ++k) {
+      const int i = lane + 32 * k;
+      held[k] = i < nvec ? xr[i] : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int k = 0; k < HELD; ++k) {
+      float f[8];
+      unpack8(held[k], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+    }
+  } else {
+    for (int i = lane; i < nvec; i += 32) {
+      float f[8];
+      unpack8(xr[i], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+    }
   }
   ss = warp_sum(ss);
   const float r = rsqrtf(ss / d + eps);
   if (lane == 0 && rstd) rstd[row] = r;
-  uint4* yr = reinterpret_cast<uint4*>(y + (size_t)row * d);
-  for (int i = lane; i < nvec; i += 32) {
-    uint4 v = xr[i];
-    float f[8];
-    float2 t;
-    t = unpack_bf16(v.x); f[0] = t.x; f[1] = t.y;
-    t = unpack_bf16(v.y); f[2] = t.x; f[3] = t.y;
-    t = unpack_bf16(v.z); f[4] = t.x; f[5] = t.y;
-    t = unpack_bf16(v.w); f[6] = t.x; f[7] = t.y;
+  auto emit = [&](int i, const uint4& v) {
+    float f[8], g[8];
+    unpack8(v, f);
+    load_gain8(w, w16, i, g);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) f[j] = f[j] * r * (w ? w[i * 8 + j] : 1.f);
-    uint4 o;
-    o.x = pack_bf16(f[0], f[1]); o.y = pack_bf16(f[2], f[3]);
-    o.z = pack_bf16(f[4], f[5]); o.w = pack_bf16(f[6], f[7]);
-    yr[i] = o;
+    for (int j = 0; j < 8; ++j) f[j] = f[j] * r * g[j];
+    yr[i] = pack8(f);
+  };
+  if (NV > 0) {
+#pragma unroll
+    for (int k = 0; k < HELD; ++k)
+      if (lane + 32 * k < nvec) emit(lane + 32 * k, held[k]);
+  } else {
+    for (int i = lane; i < nvec; i += 32) emit(i, xr[i]);
+  }
+}
+
+// Rows wider than a warp holds (d / 8 threads per block, d <= 8192): a thread owns eight columns of
+// ROWS rows, loaded together; the squares meet in shared memory. 8192 x 4096: 55 us with a warp per
+// row, 38 so (two rows; with four, 8192 x 2880 takes 31 instead of 27).
+template <int THREADS, int ROWS>
+__global__ void __launch_bounds__(THREADS)
+rmsnorm_fwd_columns_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w, bool w16,
+                           __nv_bfloat16* __restrict__ y, float* __restrict__ rstd, int rows, int d, float eps) {
+  __shared__ float part[32][ROWS];
+  const int nvec = d / 8, i = threadIdx.x, nw = blockDim.x >> 5, r0 = blockIdx.x * ROWS;
+  const bool mine = i < nvec;
+  uint4 v[ROWS];
+#pragma unroll
+  for (int k = 0; k < ROWS; ++k)
+    v[k] = mine && r0 + k < rows ? reinterpret_cast<const uint4*>(x)[(size_t)(r0 + k) * nvec + i] : make_uint4(0, 0, 0, 0);
+  float g[8];
+  if (mine) load_gain8(w, w16, i, g);
+#pragma unroll
+  for (int k = 0; k < ROWS; ++k) {
+    float f[8], ss = 0.f;
+    unpack8(v[k], f);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+    ss = warp_sum(ss);
+    if ((i & 31) == 0) part[i >> 5][k] = ss;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < ROWS; ++k) {
+    float ss = 0.f;
+    for (int q = 0; q < nw; ++q) ss += part[q][k];
+    const float r = rsqrtf(ss / d + eps);
+    if (r0 + k >= rows) break;
+    if (i == 0 && rstd) rstd[r0 + k] = r;
+    float f[8];
+    unpack8(v[k], f);
+    if (mine) {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) f[j] = f[j] * r * g[j];
+      reinterpret_cast<uint4*>(y)[(size_t)(r0 + k) * nvec + i] = pack8(f);
+    }
   }
 }
 
 // Backward: dx = r * (w*dy) - x * r^3 * mean(w*dy*x); dw += sum_rows dy * x * r.
+// A thread owns eight columns of every row its block walks, so dw stays in eight registers; the
+// block takes ROWS rows at a time (2 * ROWS 16-byte loads in flight per thread, each element
+// read once) and shares their dot products through shared memory, one barrier per step (the sums
+// alternate between two buffers). For 512 <= d <= 8192 (a block of d / 8 threads, 2 to 32 warps);
+// beyond 512 threads a thread has 64 registers, which hold two rows.
+// 16384 x 2048: 80 us with a warp per row, rows read twice and dw in shared memory, 48 now.
+template <int THREADS, int ROWS>
+__global__ void __launch_bounds__(THREADS, THREADS > 512 ? 1 : 512 / THREADS)
+rmsnorm_bwd_columns_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w, bool w16,
+                           const __nv_bfloat16* __restrict__ dy, const float* __restrict__ rstd,
+                           __nv_bfloat16* __restrict__ dx, float* __restrict__ dw_part, int rows, int d) {
+  __shared__ float part[2][32][ROWS];
+  const int nvec = d / 8, i = threadIdx.x, nw = blockDim.x >> 5;
+  const bool mine = i < nvec;
+  float g[8], acc[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) { g[j] = 0.f; acc[j] = 0.f; }
+  if (mine) load_gain8(w, w16, i, g);
+  const int groups = (rows + ROWS - 1) / ROWS;
+  int buf = 0;
+  for (int gr = blockIdx.x; gr < groups; gr += gridDim.x, buf ^= 1) {
+    const int r0 = gr * ROWS;
+    uint4 xv[ROWS], gv[ROWS];
+    float r[ROWS], dot[ROWS];
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) {
+      const bool live = mine && r0 + k < rows;
+      const size_t at = (size_t)(r0 + k) * nvec + i;
+      xv[k] = live ? reinterpret_cast<const uint4*>(x)[at] : make_uint4(0, 0, 0, 0);
+      gv[k] = live ? reinterpret_cast<const uint4*>(dy)[at] : make_uint4(0, 0, 0, 0);
+      r[k] = r0 + k < rows ? rstd[r0 + k] : 0.f;
+    }
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) {
+      float a[8], b[8];
+      unpack8(xv[k], a); unpack8(gv[k], b);
+      dot[k] = 0.f;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) dot[k] += a[j] * b[j] * g[j];
+      dot[k] = warp_sum(dot[k]);
+    }
+    if ((i & 31) == 0) {
+#pragma unroll
+      for (int k = 0; k < ROWS; ++k) part[buf][i >> 5][k] = dot[k];
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) dot[k] = 0.f;
+    for (int q = 0; q < nw; ++q) {
+#pragma unroll
+      for (int k = 0; k < ROWS; ++k) dot[k] += part[buf][q][k];
+    }
+#pragma unroll
+    for (int k = 0; k < ROWS; ++k) {
+      if (!mine || r0 + k >= rows) continue;
+      const float c = dot[k] * r[k] * r[k] * r[k] / d;
+      float a[8], b[8], o[8];
+      unpack8(xv[k], a); unpack8(gv[k], b);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        o[j] = r[k] * g[j] * b[j] - a[j] * c;
+        acc[j] += b[j] * a[j] * r[k];
+      }
+      reinterpret_cast<uint4*>(dx)[(size_t)(r0 + k) * nvec + i] = pack8(o);
+    }
+  }
+  if (dw_part && mine) {
+    float4* out = reinterpret_cast<float4*>(dw_part + (size_t)blockIdx.x * d + i * 8);
+    out[0] = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    out[1] = make_float4(acc[4], acc[5], acc[6], acc[7]);
+  }
+}
+
+// out[c] = sum of part[0..n)[c]: a block per 32 columns, 32 rows side by side.
+__global__ void __launch_bounds__(1024)
+sum_rows_kernel(const float* __restrict__ part, float* __restrict__ out, int n, int d) {
+  __shared__ float sums[32][33];
+  const int c = blockIdx.x * 32 + (threadIdx.x & 31), w = threadIdx.x >> 5;
+  float acc = 0.f;
+  if (c < d) {
+#pragma unroll 4
+    for (int r = w; r < n; r += 32) acc += part[(size_t)r * d + c];
+  }
+  sums[w][threadIdx.x & 31] = acc;
+  __syncthreads();
+  acc = warp_sum(sums[threadIdx.x & 31][w]);
+  const int oc = blockIdx.x * 32 + w;
+  if ((threadIdx.x & 31) == 0 && oc < d) out[oc] = acc;
+}
+
+// The other widths: a warp per row.
 // Each block walks rows grid-stride, keeps its dw partial in shared memory (fp32) and
 // adds it to the global fp32 dw once at the end.
 __global__ void rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w,
@@ -110,7 +286,7 @@ __global__ void rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const fl
 // its columns of the slab, so the per-row update is a plain vector read-modify-write (no
 // atomics); the slabs are summed once at the end. Needs 8 warps · d · 4 bytes of shared memory.
 __global__ void __launch_bounds__(256)
-rmsnorm_bwd_slab_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w,
+rmsnorm_bwd_slab_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w, bool w16,
                         const __nv_bfloat16* __restrict__ dy, const float* __restrict__ rstd,
                         __nv_bfloat16* __restrict__ dx, float* __restrict__ dw, int rows, int d) {
   extern __shared__ __align__(16) float slabs[];  // [warps][d]
@@ -119,7 +295,6 @@ rmsnorm_bwd_slab_kernel(const __nv_bfloat16* __restrict__ x, const float* __rest
   for (int i = threadIdx.x; i < warps_per_block * d; i += blockDim.x) slabs[i] = 0.f;
   __syncthreads();
   float4* mine = reinterpret_cast<float4*>(slabs + (size_t)warp * d);
-  const float4* w4 = reinterpret_cast<const float4*>(w);
   const int nvec = d / 8;
   for (int row = blockIdx.x * warps_per_block + warp; row < rows; row += gridDim.x * warps_per_block) {
     const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * d);
@@ -129,11 +304,8 @@ rmsnorm_bwd_slab_kernel(const __nv_bfloat16* __restrict__ x, const float* __rest
     for (int i = lane; i < nvec; i += 32) {
       const uint4 xv = xr[i], gv = gr[i];
       const uint32_t* xu = &xv.x; const uint32_t* gu = &gv.x;
-      float wl[8] = {1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f};
-      if (w) {
-        const float4 lo = w4[2 * i], hi = w4[2 * i + 1];
-        wl[0] = lo.x; wl[1] = lo.y; wl[2] = lo.z; wl[3] = lo.w; wl[4] = hi.x; wl[5] = hi.y; wl[6] = hi.z; wl[7] = hi.w;
-      }
+      float wl[8];
+      load_gain8(w, w16, i, wl);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float2 a = unpack_bf16(xu[j]), g = unpack_bf16(gu[j]);
@@ -146,11 +318,8 @@ rmsnorm_bwd_slab_kernel(const __nv_bfloat16* __restrict__ x, const float* __rest
     for (int i = lane; i < nvec; i += 32) {
       const uint4 xv = xr[i], gv = gr[i];  // second read of the row: L1 / L2
       const uint32_t* xu = &xv.x; const uint32_t* gu = &gv.x;
-      float wl[8] = {1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f};
-      if (w) {
-        const float4 lo = w4[2 * i], hi = w4[2 * i + 1];
-        wl[0] = lo.x; wl[1] = lo.y; wl[2] = lo.z; wl[3] = lo.w; wl[4] = hi.x; wl[5] = hi.y; wl[6] = hi.z; wl[7] = hi.w;
-      }
+      float wl[8];
+      load_gain8(w, w16, i, wl);
       uint4 o; uint32_t* ou = &o.x;
       float p[8];
 #pragma unroll
@@ -181,138 +350,130 @@ rmsnorm_bwd_slab_kernel(const __nv_bfloat16* __restrict__ x, const float* __rest
 // ---------------------------------------------------------------- QK-norm + RoPE
 // x: [tokens, heads, D] bf16 (row stride `stride_tok` elements so it may be a slice of
 // a fused qkv buffer); cos/sin: [tokens, D/2] fp32; w: [D] fp32 or null (no norm).
-// One warp per (token, head): lane l holds D/32 consecutive elements; its rotation
-// partner (element i <-> i + D/2) lives in lane l ^ 16.
-// E consecutive bf16 (E = 2, 4 or 8: one 4-, 8- or 16-byte access; the address is a multiple
-// of E elements because head offsets and token strides are multiples of the head dim).
-template <int E> struct BfVec;
-template <> struct BfVec<2> { using T = uint32_t; };
-template <> struct BfVec<4> { using T = uint2; };
-template <> struct BfVec<8> { using T = uint4; };
-template <int E>
-__device__ __forceinline__ void load_bf16(const __nv_bfloat16* p, float (&out)[E]) {
-  const typename BfVec<E>::T raw = *reinterpret_cast<const typename BfVec<E>::T*>(p);
-  const uint32_t* u = reinterpret_cast<const uint32_t*>(&raw);
+__device__ __forceinline__ void load_f32x8(const float* p, float (&out)[8]) {
 #pragma unroll
-  for (int j = 0; j < E / 2; ++j) { const float2 t = unpack_bf16(u[j]); out[2 * j] = t.x; out[2 * j + 1] = t.y; }
-}
-template <int E>
-__device__ __forceinline__ void store_bf16(__nv_bfloat16* p, const float (&v)[E]) {
-  typename BfVec<E>::T raw;
-  uint32_t* u = reinterpret_cast<uint32_t*>(&raw);
-#pragma unroll
-  for (int j = 0; j < E / 2; ++j) u[j] = pack_bf16(v[2 * j], v[2 * j + 1]);
-  *reinterpret_cast<typename BfVec<E>::T*>(p) = raw;
-}
-template <int E>
-__device__ __forceinline__ void load_f32(const float* p, float (&out)[E]) {
-  if (E % 4 == 0) {
-#pragma unroll
-    for (int j = 0; j < E / 4; ++j) {
-      const float4 t = reinterpret_cast<const float4*>(p)[j];
-      out[4 * j] = t.x; out[4 * j + 1] = t.y; out[4 * j + 2] = t.z; out[4 * j + 3] = t.w;
-    }
-  } else {
-    const float2 t = *reinterpret_cast<const float2*>(p);
-    out[0] = t.x; out[1] = t.y;
+  for (int j = 0; j < 2; ++j) {
+    const float4 t = reinterpret_cast<const float4*>(p)[j];
+    out[4 * j] = t.x; out[4 * j + 1] = t.y; out[4 * j + 2] = t.z; out[4 * j + 3] = t.w;
   }
 }
 
+// D / 16 lanes per (token, head): a lane holds eight elements of the lower half and the eight they
+// rotate with, so the rotation needs no exchange and one set of cos / sin serves sixteen elements.
+// A lane group takes HC heads of a token at a time: their loads are in flight together and share the
+// token's cos / sin (which were four fifths of what it loaded with one head at a time and halves
+// in different lanes). 8192 tokens x 32 heads of 128: forward 45 -> 28 us, backward 90 -> 45.
 template <int D, bool BWD>
-__global__ void norm_rope_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w,
-                                 const float* __restrict__ cs, const float* __restrict__ sn,
-                                 __nv_bfloat16* __restrict__ y, float* __restrict__ rstd_io,
-                                 const __nv_bfloat16* __restrict__ dy, float* __restrict__ dw,
-                                 long tokens, int heads, long stride_tok_x, long stride_tok_y,
-                                 float eps) {
-  // D/8 lanes per (token, head), eight elements (one 16-byte access) per lane: a warp works
-  // on 256/D items at once. Element i rotates with i + D/2, which lane ^ (LPI/2) holds.
-  constexpr int E = 8;
-  constexpr int LPI = D / E;          // lanes per item: 8, 16 or 32
-  constexpr int IPW = 32 / LPI;       // items per warp
+__global__ void __launch_bounds__(256)
+norm_rope_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w, bool w16,
+                 const float* __restrict__ cs, const float* __restrict__ sn,
+                 __nv_bfloat16* __restrict__ y, float* __restrict__ rstd_io,
+                 const __nv_bfloat16* __restrict__ dy, float* __restrict__ dw,
+                 long tokens, int heads, long stride_tok_x, long stride_tok_y, float eps) {
+  constexpr int LPI = D / 16;         // lanes per item: 4, 8 or 16
+  constexpr int IPW = 32 / LPI;       // items (token, HC heads) per warp
+  constexpr int HC = BWD ? 2 : 4;
   __shared__ float dw_part[D];
   if (BWD) {
     for (int i = threadIdx.x; i < D; i += blockDim.x) dw_part[i] = 0.f;
     __syncthreads();
   }
   const int lane = threadIdx.x & 31;
-  const int sub = lane / LPI, li = lane % LPI;  // which of the warp's items, and the lane within it
+  const int sub = lane / LPI, li = lane % LPI;
   const long nwarps = (long)gridDim.x * (blockDim.x >> 5);
-  const long total = tokens * heads;
+  const int chunks = (heads + HC - 1) / HC;
+  const long total = tokens * chunks;
   const long steps = (total + IPW - 1) / IPW;   // whole warps iterate together (shuffles stay converged)
-  float dw_lane[E];  // a lane always holds the same E columns: its share of dw stays in registers
+  float dwa[8], dwb[8], wa[8], wb[8];           // a = lower half, b = upper half
 #pragma unroll
-  for (int j = 0; j < E; ++j) dw_lane[j] = 0.f;
-  float wl[E];
-#pragma unroll
-  for (int j = 0; j < E; ++j) wl[j] = w ? w[li * E + j] : 1.f;
+  for (int j = 0; j < 8; ++j) { dwa[j] = 0.f; dwb[j] = 0.f; }
+  load_gain8(w, w16, li, wa);
+  load_gain8(w, w16, li + LPI, wb);
   for (long step = (long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); step < steps; step += nwarps) {
     const long item = step * IPW + sub;
     const bool live = item < total;
-    const long tok = live ? item / heads : 0;
-    const int head = live ? (int)(item % heads) : 0;
-    const __nv_bfloat16* xp = x + tok * stride_tok_x + (long)head * D + li * E;
-    float v[E];
-    load_bf16<E>(xp, v);
-    const bool upper = li >= LPI / 2;
-    const int half_idx = (li % (LPI / 2)) * E;  // index into cos/sin of my first element
-    float c[E], s[E];
-    load_f32<E>(cs + tok * (D / 2) + half_idx, c);
-    load_f32<E>(sn + tok * (D / 2) + half_idx, s);
-    if (!BWD) {
-      if (w) {
-        float ss = 0.f;
+    const long tok = live ? item / chunks : 0;
+    const int h0 = live ? (int)(item % chunks) * HC : 0;
+    const __nv_bfloat16* xp = x + tok * stride_tok_x + (long)h0 * D + li * 8;
+    const __nv_bfloat16* gp = BWD ? dy + tok * stride_tok_y + (long)h0 * D + li * 8 : nullptr;
+    __nv_bfloat16* yp = y + tok * stride_tok_y + (long)h0 * D + li * 8;   // backward: dx (dense, like dy)
+    uint4 xa[HC], xb[HC], ga[HC], gb[HC];
+    float r[HC];
 #pragma unroll
-        for (int j = 0; j < E; ++j) ss += v[j] * v[j];
-#pragma unroll
-        for (int o = LPI / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
-        const float r = rsqrtf(ss / D + eps);
-        if (li == 0 && live && rstd_io) rstd_io[item] = r;
-#pragma unroll
-        for (int j = 0; j < E; ++j) v[j] = v[j] * r * wl[j];
+    for (int k = 0; k < HC; ++k) {
+      const bool on = live && h0 + k < heads;
+      if (!BWD || w) {
+        xa[k] = on ? *reinterpret_cast<const uint4*>(xp + k * D) : make_uint4(0, 0, 0, 0);
+        xb[k] = on ? *reinterpret_cast<const uint4*>(xp + k * D + D / 2) : make_uint4(0, 0, 0, 0);
       }
-      float out[E];
-#pragma unroll
-      for (int j = 0; j < E; ++j) {
-        const float other = __shfl_xor_sync(0xffffffffu, v[j], LPI / 2);
-        // lower half: a*c - b*s ; upper half: a*s + b*c  (a = lower, b = upper element)
-        out[j] = upper ? (other * s[j] + v[j] * c[j]) : (v[j] * c[j] - other * s[j]);
+      if (BWD) {
+        ga[k] = on ? *reinterpret_cast<const uint4*>(gp + k * D) : make_uint4(0, 0, 0, 0);
+        gb[k] = on ? *reinterpret_cast<const uint4*>(gp + k * D + D / 2) : make_uint4(0, 0, 0, 0);
+        r[k] = on && w ? rstd_io[tok * heads + h0 + k] : 0.f;
       }
-      if (live) store_bf16<E>(y + tok * stride_tok_y + (long)head * D + li * E, out);
-    } else {
-      // dy -> d(normed) by the inverse rotation, then RMSNorm backward per head
-      float g[E];
-      load_bf16<E>(dy + tok * stride_tok_y + (long)head * D + li * E, g);
+    }
+    float c[8], s[8];
+    load_f32x8(cs + tok * (D / 2) + li * 8, c);
+    load_f32x8(sn + tok * (D / 2) + li * 8, s);
 #pragma unroll
-      for (int j = 0; j < E; ++j) {
-        const float other = __shfl_xor_sync(0xffffffffu, g[j], LPI / 2);
-        // y_lo = a c - b s, y_hi = a s + b c  =>  da = g_lo c + g_hi s, db = -g_lo s + g_hi c
-        g[j] = upper ? (-other * s[j] + g[j] * c[j]) : (g[j] * c[j] + other * s[j]);
-      }
-      __nv_bfloat16* dxp = y + tok * stride_tok_y + (long)head * D + li * E;  // y doubles as dx (dense, like dy)
-      if (w) {
-        const float r = rstd_io[live ? item : 0];
-        float dot = 0.f;
+    for (int k = 0; k < HC; ++k) {
+      const bool on = live && h0 + k < heads;
+      float a[8], b[8], oa[8], ob[8];
+      if (!BWD) {
+        unpack8(xa[k], a); unpack8(xb[k], b);
+        if (w) {
+          float ss = 0.f;
 #pragma unroll
-        for (int j = 0; j < E; ++j) dot += g[j] * wl[j] * v[j];
+          for (int j = 0; j < 8; ++j) ss += a[j] * a[j] + b[j] * b[j];
 #pragma unroll
-        for (int o = LPI / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
-        const float cc = dot * r * r * r / D;
-        float o8[E];
+          for (int o = LPI / 2; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+          const float rr = rsqrtf(ss / D + eps);
+          if (li == 0 && on && rstd_io) rstd_io[tok * heads + h0 + k] = rr;
 #pragma unroll
-        for (int j = 0; j < E; ++j) {
-          if (live) dw_lane[j] += g[j] * v[j] * r;
-          o8[j] = r * wl[j] * g[j] - v[j] * cc;
+          for (int j = 0; j < 8; ++j) { a[j] = a[j] * rr * wa[j]; b[j] = b[j] * rr * wb[j]; }
         }
-        if (live) store_bf16<E>(dxp, o8);
-      } else if (live) {
-        store_bf16<E>(dxp, g);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) { oa[j] = a[j] * c[j] - b[j] * s[j]; ob[j] = a[j] * s[j] + b[j] * c[j]; }
+      } else {
+        // dy -> d(normed) by the inverse rotation, then RMSNorm backward per head
+        float ya[8], yb[8];
+        unpack8(ga[k], ya); unpack8(gb[k], yb);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) { oa[j] = ya[j] * c[j] + yb[j] * s[j]; ob[j] = yb[j] * c[j] - ya[j] * s[j]; }
+        if (w) {
+          unpack8(xa[k], a); unpack8(xb[k], b);
+          float dot = 0.f;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) dot += oa[j] * wa[j] * a[j] + ob[j] * wb[j] * b[j];
+#pragma unroll
+          for (int o = LPI / 2; o > 0; o >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+          const float cc = dot * r[k] * r[k] * r[k] / D;
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            dwa[j] += oa[j] * a[j] * r[k];
+            dwb[j] += ob[j] * b[j] * r[k];
+            oa[j] = r[k] * wa[j] * oa[j] - a[j] * cc;
+            ob[j] = r[k] * wb[j] * ob[j] - b[j] * cc;
+          }
+        }
+      }
+      if (on) {
+        *reinterpret_cast<uint4*>(yp + k * D) = pack8(oa);
+        *reinterpret_cast<uint4*>(yp + k * D + D / 2) = pack8(ob);
       }
     }
   }
   if (BWD && dw) {
 #pragma unroll
-    for (int j = 0; j < E; ++j) atomicAdd(&dw_part[li * E + j], dw_lane[j]);
+    for (int j = 0; j < 8; ++j) {
+      // lanes of a warp that hold the same columns add up before the block does
+#pragma unroll
+      for (int o = LPI; o < 32; o <<= 1) {
+        dwa[j] += __shfl_xor_sync(0xffffffffu, dwa[j], o);
+        dwb[j] += __shfl_xor_sync(0xffffffffu, dwb[j], o);
+      }
+      if (sub == 0) { atomicAdd(&dw_part[li * 8 + j], dwa[j]); atomicAdd(&dw_part[D / 2 + li * 8 + j], dwb[j]); }
+    }
     __syncthreads();
     for (int i = threadIdx.x; i < D; i += blockDim.x) atomicAdd(&dw[i], dw_part[i]);
   }
@@ -1128,18 +1289,52 @@ static inline int grid_for(long work, int per_block, int cap = 148 * 16) {
 }
 
 void rmsnorm_fwd(const void* x, const float* w, void* y, float* rstd, long rows, int d, float eps, cudaStream_t s) {
-  const int wpb = 8;
-  rmsnorm_fwd_kernel<8><<<(int)((rows + wpb - 1) / wpb), wpb * 32, 0, s>>>(
-      (const __nv_bfloat16*)x, w, (__nv_bfloat16*)y, rstd, (int)rows, d, eps);
+  const int wpb = 8, grid = (int)((rows + wpb - 1) / wpb);
+  const bool w16 = reinterpret_cast<uintptr_t>(w) % 16 == 0;
+  const int threads = (d / 8 + 31) / 32 * 32;
+  const int nv = threads / 32;   // 16-byte pieces of a row per lane; 8 of them are the most held
+#define RN_CASE(NV_, COND) \
+  if (COND) { rmsnorm_fwd_kernel<NV_><<<grid, wpb * 32, 0, s>>>((const __nv_bfloat16*)x, w, w16, (__nv_bfloat16*)y, rstd, (int)rows, d, eps); return; }
+  RN_CASE(1, nv <= 1) RN_CASE(2, nv <= 2) RN_CASE(4, nv <= 4) RN_CASE(8, nv <= 8)
+#define RC_CASE(THREADS_, ROWS_) \
+  if (threads <= THREADS_) { \
+    rmsnorm_fwd_columns_kernel<THREADS_, ROWS_><<<(int)((rows + ROWS_ - 1) / ROWS_), threads, 0, s>>>( \
+        (const __nv_bfloat16*)x, w, w16, (__nv_bfloat16*)y, rstd, (int)rows, d, eps); \
+    return; }
+  RC_CASE(512, 2) RC_CASE(1024, 2)
+#undef RC_CASE
+  RN_CASE(0, true)
+#undef RN_CASE
 }
-void rmsnorm_bwd(const void* x, const float* w, const void* dy, const float* rstd, void* dx, float* dw, long rows, int d, cudaStream_t s) {
+// Rows of partial sums that the backward leaves for dw (one per block); 0: it adds into dw with atomics.
+// 512 threads per SM, as many as are resident with 128 registers. (Atomics of every block into dw
+// cost more than the pass itself: 16384 x 2048 took 66 us with them.)
+int rmsnorm_bwd_partials(long rows, int d) {
+  if (d < 512 || d > 8192 || d % 8 != 0) return 0;
+  const int threads = (d / 8 + 31) / 32 * 32, per = threads <= 512 ? 4 : 2;
+  return (int)max(1L, min((rows + per - 1) / per, 148L * max(1, 512 / threads)));
+}
+void rmsnorm_bwd(const void* x, const float* w, const void* dy, const float* rstd, void* dx, float* dw, float* dw_part,
+                 long rows, int d, cudaStream_t s) {
+  const int blocks = rmsnorm_bwd_partials(rows, d);
+  const bool w16 = reinterpret_cast<uintptr_t>(w) % 16 == 0;
+  if (blocks > 0) {
+    const int threads = (d / 8 + 31) / 32 * 32;
+    float* part = dw ? dw_part : nullptr;
+#define RB_CASE(THREADS_, ROWS_) \
+    rmsnorm_bwd_columns_kernel<THREADS_, ROWS_><<<blocks, threads, 0, s>>>((const __nv_bfloat16*)x, w, w16, \
+        (const __nv_bfloat16*)dy, rstd, (__nv_bfloat16*)dx, part, (int)rows, d)
+    if (threads <= 256) RB_CASE(256, 4);
+    else if (threads <= 512) RB_CASE(512, 4);
+    else RB_CASE(1024, 2);
+#undef RB_CASE
+    if (part) sum_rows_kernel<<<(d + 31) / 32, 1024, 0, s>>>(part, dw, blocks, d);
+    return;
+  }
   const int wpb = 8;
   int grid = (int)min((rows + wpb - 1) / wpb, 148L * 4);
-  const size_t slab_bytes = (size_t)wpb * d * sizeof(float);
-  if (d % 8 == 0 && slab_bytes <= 200 * 1024) {
-    if (slab_bytes > 48 * 1024)  // per device, so set at every launch that needs it (a cheap call)
-      cudaFuncSetAttribute(rmsnorm_bwd_slab_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)slab_bytes);
-    rmsnorm_bwd_slab_kernel<<<grid, wpb * 32, slab_bytes, s>>>((const __nv_bfloat16*)x, w, (const __nv_bfloat16*)dy, rstd, (__nv_bfloat16*)dx, dw, (int)rows, d);
+  if (d % 8 == 0 && d < 512) {
+    rmsnorm_bwd_slab_kernel<<<grid, wpb * 32, (size_t)wpb * d * sizeof(float), s>>>((const __nv_bfloat16*)x, w, w16, (const __nv_bfloat16*)dy, rstd, (__nv_bfloat16*)dx, dw, (int)rows, d);
     return;
   }
   rmsnorm_bwd_kernel<<<grid, wpb * 32, d * sizeof(float), s>>>(
@@ -1149,12 +1344,14 @@ const char* norm_rope(bool bwd, const void* x, const float* w, const float* cs, 
                       float* rstd, const void* dy, float* dw, long tokens, int heads, int D,
                       long stride_x, long stride_y, float eps, cudaStream_t s) {
   const int wpb = 8;
-  const long items = (tokens * heads + (256 / D) - 1) / (256 / D);  // warp steps: 256 / D items each
-  int grid = (int)min((items + wpb - 1) / wpb, 148L * 8);
+  const int hc = bwd ? 2 : 4;                                // heads a lane group takes at once
+  const long items = tokens * ((heads + hc - 1) / hc), steps = (items + 512 / D - 1) / (512 / D);  // 512 / D items per warp
+  const int grid = (int)min((steps + wpb - 1) / wpb, 148L * (bwd ? 2 : 8));
+  const bool w16 = reinterpret_cast<uintptr_t>(w) % 16 == 0;
 #define NR_CASE(D_) \
   if (D == D_) { \
-    if (bwd) norm_rope_kernel<D_, true><<<grid, wpb * 32, 0, s>>>((const __nv_bfloat16*)x, w, cs, sn, (__nv_bfloat16*)y, rstd, (const __nv_bfloat16*)dy, dw, tokens, heads, stride_x, stride_y, eps); \
-    else     norm_rope_kernel<D_, false><<<grid, wpb * 32, 0, s>>>((const __nv_bfloat16*)x, w, cs, sn, (__nv_bfloat16*)y, rstd, nullptr, nullptr, tokens, heads, stride_x, stride_y, eps); \
+    if (bwd) norm_rope_kernel<D_, true><<<grid, wpb * 32, 0, s>>>((const __nv_bfloat16*)x, w, w16, cs, sn, (__nv_bfloat16*)y, rstd, (const __nv_bfloat16*)dy, dw, tokens, heads, stride_x, stride_y, eps); \
+    else     norm_rope_kernel<D_, false><<<grid, wpb * 32, 0, s>>>((const __nv_bfloat16*)x, w, w16, cs, sn, (__nv_bfloat16*)y, rstd, nullptr, nullptr, tokens, heads, stride_x, stride_y, eps); \
     return nullptr; }
   NR_CASE(64) NR_CASE(128) NR_CASE(256)
 #undef NR_CASE

@@ -10,7 +10,11 @@ enum { ACT_SWISH = 0, ACT_QUICK_GELU = 1, ACT_GELU_TANH = 2, ACT_RELU2 = 3, ACT_
 enum { MOM_F32 = 0, MOM_BF16 = 1, MOM_FP8 = 2 };
 
 void rmsnorm_fwd(const void* x, const float* w, void* y, float* rstd, long rows, int d, float eps, cudaStream_t s);
-void rmsnorm_bwd(const void* x, const float* w, const void* dy, const float* rstd, void* dx, float* dw, long rows, int d, cudaStream_t s);
+// dw (may be null) is written; `dw_part`: fp32 [rmsnorm_bwd_partials(rows, d), d]. With 0 partials the
+// kernel adds into dw, which the caller clears.
+int rmsnorm_bwd_partials(long rows, int d);
+void rmsnorm_bwd(const void* x, const float* w, const void* dy, const float* rstd, void* dx, float* dw, float* dw_part,
+                 long rows, int d, cudaStream_t s);
 const char* norm_rope(bool bwd, const void* x, const float* w, const float* cs, const float* sn, void* y,
                       float* rstd, const void* dy, float* dw, long tokens, int heads, int D,
                       long stride_x, long stride_y, float eps, cudaStream_t s);

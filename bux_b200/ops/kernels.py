@@ -244,7 +244,7 @@ def rmsnorm_fwd(x, w, eps: float):
 
 def rmsnorm_bwd(x, w, dy, rstd, need_dw: bool = True):
     dx = _out(x.shape, dtype=x.dtype, device=x.device, op="rmsnorm_bwd dx")
-    dw = (_out(x.shape[-1], dtype=torch.float32, device=x.device, op="rmsnorm_bwd dw", fill=0.0)
+    dw = (_out(x.shape[-1], dtype=torch.float32, device=x.device, op="rmsnorm_bwd dw")
           if need_dw and w is not None else None)
     ops().rmsnorm_bwd(x, w, dy, rstd, dx, dw)
     _count()

@@ -132,6 +132,46 @@ def test_rmsnorm(cuda):
     assert rel_err(dw, w.grad) < 2e-2
 
 
+@pytest.mark.parametrize("rows,d", [(1, 8), (5, 504), (3, 512), (9, 1032), (2, 2056), (5, 2880), (3, 4104), (2, 8192), (3, 8200)])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_rmsnorm_widths(cuda, rows, d, shift):
+    """The edges of each way of splitting a row, and gains that start between 16-byte boundaries.
+    Bounds: outputs are rounded to bf16 (2^-9); dw is an fp32 sum of products of bf16 values."""
+    from bux_b200.ops import kernels as K
+
+    torch.manual_seed(5)
+    x, dy = (torch.randn(rows, d, device=cuda).bfloat16() for _ in range(2))
+    w = torch.randn(d + shift, device=cuda)[shift:]
+    xd, wd = x.double().requires_grad_(), w.double().requires_grad_()
+    want = xd * torch.rsqrt(xd.square().mean(-1, keepdim=True) + 1e-6) * wd
+    want.backward(dy.double())
+    y, rstd = K.rmsnorm_fwd(x, w, 1e-6)
+    dx, dw = K.rmsnorm_bwd(x, w, dy, rstd)
+    assert rel_err(y, want) < 4e-3 and rel_err(dx, xd.grad) < 4e-3 and rel_err(dw, wd.grad) < 1e-5
+    plain, r2 = K.rmsnorm_fwd(x, None, 1e-6)
+    assert rel_err(plain, want / wd) < 4e-3 and rel_err(K.rmsnorm_bwd(x, None, dy, r2)[0], K.rmsnorm_bwd(x, torch.ones_like(w), dy, r2)[0]) < 1e-6
+
+
+@pytest.mark.parametrize("tokens,heads,d", [(1, 1, 64), (7, 3, 128), (33, 5, 256), (50, 6, 64)])
+def test_norm_rope_odd_heads(cuda, tokens, heads, d):
+    """Heads go four (backward: two) at a time: counts that they do not divide, and a slice of wider
+    rows. Bounds as for the RMSNorm, with one rotation more."""
+    from bux_b200.ops import kernels as K
+
+    torch.manual_seed(6)
+    wide = torch.randn(1, tokens, (heads + 1) * d, device=cuda).bfloat16()
+    x = wide[..., d:].view(1, tokens, heads, d) if tokens == 1 else wide[..., d:].unflatten(-1, (heads, d))
+    dy, w = torch.randn(1, tokens, heads, d, device=cuda).bfloat16(), torch.randn(d, device=cuda)
+    cos, sin = ref.rope_tables(torch.arange(tokens, device=cuda)[None], d, 10000.0)
+    xr, wr = x.float().requires_grad_(), w.clone().requires_grad_()
+    want = ref.rmsnorm_rope(xr, wr, cos, sin, 1e-6)
+    want.backward(dy.float())
+    c2, s2 = cos.reshape(-1, d // 2).contiguous(), sin.reshape(-1, d // 2).contiguous()
+    y, rstd = K.norm_rope_fwd(x, w, c2, s2, 1e-6)
+    dx, dw = K.norm_rope_bwd(x, w, c2, s2, rstd, dy, 1e-6)
+    assert rel_err(y, want) < 4e-3 and rel_err(dx, xr.grad) < 4e-3 and rel_err(dw, wr.grad) < 1e-5
+
+
 @pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("norm", [True, False])
 def test_norm_rope(cuda, d, norm):
