@@ -204,6 +204,17 @@ void ce_fwd_bwd(Tensor& logits, const Tensor& targets, const c10::optional<Tenso
   bux::ce_fwd_bwd(logits.data_ptr(), targets.data_ptr<int>(), opt_f32(mask), loss.data_ptr<float>(), lz,
                   logits.size(0), (int)logits.size(1), logits.stride(0), (float)grad_scale, (float)z_weight, (float)softcap, stream_of(logits));
 }
+void scale_to_bf16(const Tensor& src, const Tensor& scale, Tensor& out) {
+  check_cuda(src, "src"); check_cuda(out, "out");
+  TORCH_CHECK((src.scalar_type() == at::kFloat || src.scalar_type() == at::kBFloat16) && out.scalar_type() == at::kBFloat16 &&
+              out.numel() == src.numel(), "scale_to_bf16: fp32 or bf16 into bf16 of the same size");
+  TORCH_CHECK(scale.is_cuda() && scale.scalar_type() == at::kFloat && scale.numel() == 1, "scale_to_bf16: the scale is one fp32 value on the device");
+  TORCH_CHECK(reinterpret_cast<uintptr_t>(src.data_ptr()) % 16 == 0 && reinterpret_cast<uintptr_t>(out.data_ptr()) % 16 == 0,
+              "scale_to_bf16: 16-byte aligned buffers");
+  if (src.numel() == 0) return;
+  c10::cuda::CUDAGuard guard(src.device());
+  bux::scale_to_bf16(src.data_ptr(), src.scalar_type() == at::kBFloat16, scale.data_ptr<float>(), out.data_ptr(), src.numel(), stream_of(src));
+}
 void adamw(Tensor& p, const Tensor& g, Tensor& m, Tensor& v, const c10::optional<Tensor>& m_sf,
            const c10::optional<Tensor>& v_sf, const c10::optional<Tensor>& shadow,
            const c10::optional<Tensor>& grad_scale, double lr, double b1, double b2, double eps,
@@ -518,6 +529,7 @@ TORCH_LIBRARY(bux_b200, m) {
   m.def("quant_mxfp8(Tensor x, Tensor? row_index, Tensor? row_scale, Tensor? q_row, Tensor? sf_row, Tensor? q_col, Tensor? sf_col, int rows, int cols, int ld_col, int batch, int x_batch_stride) -> ()", &quant_mxfp8);
   m.def("quant_mxfp8_glu(Tensor h, Tensor? dout, Tensor? row_scale, Tensor? q_row, Tensor? sf_row, Tensor? q_col, Tensor? sf_col, int ld_col, int kind, float limit, float up_offset) -> ()", &quant_mxfp8_glu);
   m.def("quant_nvfp4(Tensor x, Tensor tensor_scale, Tensor(a!) packed, Tensor(b!) scales) -> ()", &quant_nvfp4);
+  m.def("scale_to_bf16(Tensor src, Tensor scale, Tensor(a!) out) -> ()", &scale_to_bf16);
   m.def("ce_fwd_bwd(Tensor(a!) logits, Tensor targets, Tensor? mask, Tensor(b!) loss, Tensor? logz, float grad_scale, float z_weight, float softcap) -> ()", &ce_fwd_bwd);
   m.def("adamw(Tensor(a!) p, Tensor g, Tensor(b!) m, Tensor(c!) v, Tensor? m_sf, Tensor? v_sf, Tensor? shadow, Tensor? grad_scale, float lr, float b1, float b2, float eps, float wd, float bc1, float bc2, float grad_scale_const) -> ()", &adamw);
   m.def("sumsq(Tensor g, Tensor(a!) out) -> ()", &sumsq);

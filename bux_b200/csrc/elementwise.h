@@ -35,6 +35,8 @@ void requant_mxfp8_cols(const uint8_t* q, const uint8_t* sf, uint8_t* q_col, uin
 void quant_nvfp4(const void* x, const float* tensor_scale, uint8_t* packed, uint8_t* scales, long rows, int cols,
                  cudaStream_t s);
 void ce_fwd_bwd(void* logits, const int* targets, const float* mask, float* loss, float* logz, long rows, int vocab, long ld, float grad_scale, float z_weight, float softcap, cudaStream_t s);
+// out (bf16) = src (fp32 or bf16) * *scale; src and out start on 16-byte boundaries
+void scale_to_bf16(const void* src, bool src_bf16, const float* scale, void* out, long n, cudaStream_t s);
 const char* adamw(void* p, bool p_bf16, const void* g, bool g_bf16, void* m, void* v, uint8_t* m_sf, uint8_t* v_sf, int mom,
                   void* shadow, long n, float lr, float b1, float b2, float eps, float wd, float bc1, float bc2,
                   const float* gscale_ptr, float gscale, cudaStream_t s);

@@ -320,6 +320,14 @@ def ce_fwd_bwd(logits, targets, mask, grad_scale: float, z_weight: float = 0.0, 
     return loss
 
 
+def scale_to_bf16(src, scale):
+    """bf16(src * scale) of fp32 or bf16 `src`, `scale` one fp32 value on the device."""
+    out = _out(src.shape, dtype=torch.bfloat16, device=src.device, op="scale_to_bf16")
+    ops().scale_to_bf16(src, scale, out)
+    _count()
+    return out
+
+
 def adamw(p, g, m, v, *, lr, b1, b2, eps, wd, step: int, m_sf=None, v_sf=None, shadow=None,
           grad_scale: Optional[torch.Tensor] = None, grad_scale_const: float = 1.0) -> None:
     ops().adamw(p, g, m, v, m_sf, v_sf, shadow, grad_scale, lr, b1, b2, eps, wd,

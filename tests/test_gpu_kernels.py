@@ -227,6 +227,44 @@ def test_cross_entropy(cuda):
     assert rel_err(work, lf.grad) < 2e-2
 
 
+@pytest.mark.parametrize("vocab", [8, 4096, 16384 + 8, 50304])
+@pytest.mark.parametrize("case", ["plain", "masked", "softcap"])
+def test_cross_entropy_rows_and_masked_logits(cuda, vocab, case):
+    """One pass keeps the maximum and the sum: rows shorter than a block's step, remainders of the
+    unrolled walk, logits of -inf and of the type's lowest value, a maximum that comes last.
+    Bounds: the loss is an fp32 sum, the gradient is rounded to bf16 (2^-9)."""
+    from bux_b200.ops import kernels as K
+
+    torch.manual_seed(8)
+    rows, cap = 5, 20.0 if case == "softcap" else 0.0
+    logits = (torch.randn(rows, vocab, device=cuda) * 4).bfloat16()
+    targets = torch.randint(0, vocab, (rows,), device=cuda, dtype=torch.int32)
+    logits[1, -1] = 60.0
+    if case == "masked":
+        logits[2, : vocab // 2] = float("-inf")
+        logits[3, 1:] = torch.finfo(torch.bfloat16).min
+        targets[2], targets[3] = vocab - 1, 0
+    z = logits.double()
+    z = cap * torch.tanh(z / cap) if cap else z
+    logp = torch.log_softmax(z, -1)
+    want = -logp.gather(1, targets.long()[:, None])[:, 0]
+    grad = logp.exp().scatter_add(1, targets.long()[:, None], -torch.ones(rows, 1, device=cuda, dtype=torch.float64))
+    grad = grad * (1 - (z / cap) ** 2) if cap else grad
+    loss = K.ce_fwd_bwd(logits, targets, None, 1.0, softcap=cap)
+    assert rel_err(loss, want) < 1e-5
+    # an entry p - 1 at the target cancels where p is near 1: its error is that of p, 2^-22
+    assert torch.allclose(logits.double(), grad, rtol=2 ** -8, atol=4e-6)
+
+
+@pytest.mark.parametrize("n", [1, 7, 8, 4099, 1 << 20])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_scale_to_bf16(cuda, n, dtype):
+    from bux_b200.ops import kernels as K
+
+    src, g = torch.randn(n, device=cuda).to(dtype), torch.tensor(0.37, device=cuda)
+    assert torch.equal(K.scale_to_bf16(src, g), (src.float() * g).bfloat16())
+
+
 @pytest.mark.parametrize("mom", ["f32", "bf16", "fp8"])
 def test_adamw(cuda, mom):
     from bux_b200.ops import kernels as K
