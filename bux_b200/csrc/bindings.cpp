@@ -246,6 +246,24 @@ void topk_rows(const Tensor& scores, Tensor& idx) {
                                    (int)scores.size(1), (int)idx.size(1), stream_of(scores));
   TORCH_CHECK(err == nullptr, err);
 }
+void sort_picks(const Tensor& experts, const c10::optional<Tensor>& weights, Tensor& row_index, Tensor& pos, Tensor& offsets,
+                const c10::optional<Tensor>& w_row, const c10::optional<Tensor>& status, int64_t align) {
+  check_cuda(experts, "experts"); check_cuda(row_index, "row_index"); check_cuda(pos, "pos"); check_cuda(offsets, "offsets");
+  const int64_t n = experts.numel(), E = offsets.numel() - 1, rows = row_index.numel();
+  TORCH_CHECK(experts.scalar_type() == at::kLong && experts.dim() == 2 && n > 0 && n < (1LL << 31), "sort_picks: int64 [t, k]");
+  TORCH_CHECK(row_index.scalar_type() == at::kInt && pos.scalar_type() == at::kInt && offsets.scalar_type() == at::kInt && pos.numel() == n,
+              "sort_picks: int32 outputs");
+  TORCH_CHECK(E >= 1 && E <= 1024 && align >= 1, "sort_picks: 1 to 1024 experts");
+  TORCH_CHECK(rows >= n + E * (align - 1), "sort_picks: too few rows for every expert's padding");
+  TORCH_CHECK(weights.has_value() == w_row.has_value(), "sort_picks: weights and their rows go together");
+  TORCH_CHECK(!weights.has_value() || weights->numel() == n, "sort_picks: a weight per pick");
+  TORCH_CHECK(!w_row.has_value() || (w_row->scalar_type() == at::kFloat && w_row->numel() == rows && w_row->is_contiguous()), "sort_picks: w_row is fp32 [rows]");
+  c10::cuda::CUDAGuard guard(experts.device());
+  Tensor work = at::empty({(bux::pick_blocks(n) + 1) * E}, offsets.options());
+  bux::sort_picks(reinterpret_cast<const long long*>(experts.data_ptr<int64_t>()), opt_f32(weights), n, (int)experts.size(1), (int)E, (int)align,
+                  row_index.data_ptr<int>(), pos.data_ptr<int>(), offsets.data_ptr<int>(), w_row.has_value() ? w_row->data_ptr<float>() : nullptr,
+                  rows, work.data_ptr<int>(), status_ptr(status), stream_of(experts));
+}
 void gather_rows(const Tensor& x, const Tensor& index, Tensor& out) {
   check_cuda(x, "x"); check_cuda(out, "out");
   c10::cuda::CUDAGuard guard(x.device());
@@ -534,6 +552,7 @@ TORCH_LIBRARY(bux_b200, m) {
   m.def("adamw(Tensor(a!) p, Tensor g, Tensor(b!) m, Tensor(c!) v, Tensor? m_sf, Tensor? v_sf, Tensor? shadow, Tensor? grad_scale, float lr, float b1, float b2, float eps, float wd, float bc1, float bc2, float grad_scale_const) -> ()", &adamw);
   m.def("sumsq(Tensor g, Tensor(a!) out) -> ()", &sumsq);
   m.def("topk_rows(Tensor scores, Tensor(a!) idx) -> ()", &topk_rows);
+  m.def("sort_picks(Tensor experts, Tensor? weights, Tensor(a!) row_index, Tensor(b!) pos, Tensor(c!) offsets, Tensor(d!)? w_row, Tensor(e!)? status, int align) -> ()", &sort_picks);
   m.def("gather_rows(Tensor x, Tensor index, Tensor(a!) out) -> ()", &gather_rows);
   m.def("combine_bwd(Tensor? y, Tensor dout, Tensor pos, Tensor? w, Tensor(a!)? dy, Tensor(b!)? dw) -> ()", &combine_bwd);
   m.def("combine_rows(Tensor y, Tensor pos, Tensor? w, Tensor(a!) out) -> ()", &combine_rows);

@@ -19,6 +19,7 @@ const char* norm_rope(bool bwd, const void* x, const float* w, const float* cs, 
                       float* rstd, const void* dy, float* dw, long tokens, int heads, int D,
                       long stride_x, long stride_y, float eps, cudaStream_t s);
 void glu_fwd(const void* h, void* out, const float* row_scale, long rows, int f, int kind, float limit, float up_offset, cudaStream_t s);
+// d_row_scale (may be null) is written
 void glu_bwd(const void* h, const void* dout, void* dh, const float* row_scale, float* d_row_scale, long rows, int f, int kind, float limit, float up_offset, cudaStream_t s);
 void quant_mxfp8(const void* x, long ld_x, const int* row_index, const float* row_scale, uint8_t* q_row, uint8_t* sf_row, uint8_t* q_col, uint8_t* sf_col, long rows, int cols, long ld_col, int batch, long x_batch_stride, cudaStream_t s);
 // Quantise glu(h) [rows, f] (dout null) or the gradient of h [rows, 2f] given dout [rows, f],
@@ -43,6 +44,12 @@ const char* adamw(void* p, bool p_bf16, const void* g, bool g_bf16, void* m, voi
 void sumsq(const void* g, bool bf16, long n, float* out, cudaStream_t s);
 // indices (int64) of the k largest entries of each fp32 row, descending; n <= 512
 const char* topk_rows(const float* scores, long* idx, long rows, int n, int k, cudaStream_t s);
+// Picks [n] in expert order (E <= 1024), padded to `align` rows per expert; see the kernels. `work`:
+// int32 [(pick_blocks(n) + 1) * E]; row_index and w_row (null without weights) have `rows` entries.
+struct Status;
+int pick_blocks(long n);
+void sort_picks(const long long* experts, const float* weights, long n, int k, int E, int align, int* row_index, int* pos,
+                int* offsets, float* w_row, long rows, int* work, Status* st, cudaStream_t s);
 void gather_rows(const void* x, const int* index, void* out, long rows, int d, cudaStream_t s);
 void combine_bwd(const void* y, const void* dout, const int* pos, const float* w, void* dy, float* dw, long picks, int k, int d, cudaStream_t s);
 // causal depthwise convolution over the tokens (conv_sm100.cu): forward (bwd = false: out = y, `in` = x) and

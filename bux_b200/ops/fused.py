@@ -13,6 +13,7 @@ from typing import Optional
 import torch
 import torch.nn.functional as F
 
+from . import functional
 from . import reference as ref
 from .functional import _K, kernels_on
 
@@ -103,8 +104,16 @@ def sort_picks(experts: torch.Tensor, num_experts: int, align: int = 128):
     Returns (row_index int32[R] = source token of each padded row or -1,
     pos int32[T,k] = padded row of each pick, offsets int32[E+1]) where
     R = T·k + E·(align-1) rounded up to `align` bounds the padded rows."""
+    return _sort_picks(experts, num_experts, align)[:3]
+
+
+def _sort_picks(experts: torch.Tensor, num_experts: int, align: int = 128, weights: Optional[torch.Tensor] = None):
+    """`sort_picks` and, with `weights` (fp32 [T, k]), the weight of each padded row (0 for padding)."""
     t, k = experts.shape
     dev = experts.device
+    r_max = -(-(t * k + num_experts * (align - 1)) // align) * align
+    if experts.is_cuda and experts.dtype == torch.int64 and experts.numel() and num_experts <= 1024 and not functional._OFF:
+        return _K().sort_picks(experts.contiguous(), num_experts, align, r_max, weights)
     flat = experts.reshape(-1)
     order = torch.argsort(flat, stable=True)
     counts = torch.bincount(flat, minlength=num_experts)
@@ -115,19 +124,16 @@ def sort_picks(experts: torch.Tensor, num_experts: int, align: int = 128):
     sorted_expert = flat[order]
     rank = torch.arange(t * k, device=dev) - starts[sorted_expert]
     dest = offsets[:-1][sorted_expert] + rank
-    r_max = -(-(t * k + num_experts * (align - 1)) // align) * align
     row_index = torch.full((r_max,), -1, dtype=torch.int32, device=dev)
     row_index[dest] = (order // k).to(torch.int32)
     pos = torch.empty(t * k, dtype=torch.int32, device=dev)
     pos[order] = dest.to(torch.int32)
-    return row_index, pos.view(t, k), offsets.to(torch.int32)
-
-
-def _row_weights(wts: torch.Tensor, pos: torch.Tensor, rows: int) -> torch.Tensor:
-    """fp32[rows]: the router weight of each expert-sorted row (0 for padding rows)."""
-    w_row = torch.zeros(rows, dtype=torch.float32, device=wts.device)
-    w_row[pos.reshape(-1).long()] = wts.reshape(-1)
-    return w_row
+    pos = pos.view(t, k)
+    w_row = None
+    if weights is not None:
+        w_row = torch.zeros(r_max, dtype=torch.float32, device=dev)
+        w_row[pos.reshape(-1).long()] = weights.reshape(-1)
+    return row_index, pos, offsets.to(torch.int32), w_row
 
 
 class _SortedExperts(torch.autograd.Function):
@@ -160,9 +166,8 @@ class _SortedExperts(torch.autograd.Function):
         saved = []
         for c in range(chunks):
             xc, ec, wc = x[c * tc:(c + 1) * tc], experts[c * tc:(c + 1) * tc], wts[c * tc:(c + 1) * tc]
-            row_index, pos, offsets = sort_picks(ec, e)
+            row_index, pos, offsets, w_row = _sort_picks(ec, e, weights=wc)
             rows = row_index.numel()
-            w_row = _row_weights(wc, pos, rows)
             xtq = xtsf = None
             if mx:
                 xq, xsf, xtq, xtsf = K.quant_mxfp8(xc, row_index=row_index, rows=rows, colwise=grad)

@@ -294,7 +294,7 @@ def glu_fwd(h, kind: str = "swish", row_scale=None, limit: float = 0.0, up_offse
 
 def glu_bwd(h, dout, kind: str = "swish", row_scale=None, limit: float = 0.0, up_offset: float = 0.0):
     dh = _out(h.shape, dtype=h.dtype, device=h.device, op="glu_bwd dh")
-    drs = (_out(row_scale.shape, dtype=row_scale.dtype, device=h.device, op="glu_bwd d_row_scale", fill=0.0)
+    drs = (_out(row_scale.shape, dtype=row_scale.dtype, device=h.device, op="glu_bwd d_row_scale")
            if row_scale is not None else None)
     ops().glu_bwd(h, dout, dh, row_scale, drs, ACT_KINDS[kind], limit or 0.0, up_offset)
     _count()
@@ -302,10 +302,8 @@ def glu_bwd(h, dout, kind: str = "swish", row_scale=None, limit: float = 0.0, up
 
 
 def glu_bwd_into(h, dout, kind: str, row_scale, d_row_scale, limit: float = 0.0, up_offset: float = 0.0):
-    """`glu_bwd` whose per-row gradient of `row_scale` lands in the caller's fp32 buffer
-    (cleared here first: the kernel adds into it). Returns dh."""
+    """`glu_bwd` whose per-row gradient of `row_scale` lands in the caller's fp32 buffer. Returns dh."""
     dh = _out(h.shape, dtype=h.dtype, device=h.device, op="glu_bwd dh")
-    d_row_scale.zero_()
     ops().glu_bwd(h, dout, dh, row_scale, d_row_scale, ACT_KINDS[kind], limit or 0.0, up_offset)
     _count()
     return dh
@@ -348,6 +346,20 @@ def topk_rows(scores: torch.Tensor, k: int) -> torch.Tensor:
     ops().topk_rows(flat, idx)
     _count()
     return idx.view(*scores.shape[:-1], k)
+
+
+def sort_picks(experts: torch.Tensor, num_experts: int, align: int, rows: int, weights=None):
+    """(row_index int32 [rows], pos int32 [t, k], offsets int32 [E + 1], w_row fp32 [rows] or None) of
+    the picks `experts` (int64 [t, k]) in expert order: see `fused.sort_picks`. A pick outside
+    [0, E) is reported in the status word and makes its token's combined row NaN."""
+    dev = experts.device
+    row_index = _out(rows, dtype=torch.int32, device=dev, op="sort_picks row_index")
+    pos = _out(experts.shape, dtype=torch.int32, device=dev, op="sort_picks pos")
+    offsets = _out(num_experts + 1, dtype=torch.int32, device=dev, op="sort_picks offsets")
+    w_row = _out(rows, dtype=torch.float32, device=dev, op="sort_picks w_row") if weights is not None else None
+    ops().sort_picks(experts, weights, row_index, pos, offsets, w_row, status_word(dev), align)
+    _count(3)
+    return row_index, pos, offsets, w_row
 
 
 def gather_rows(x, index, rows: int):

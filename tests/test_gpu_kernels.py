@@ -308,6 +308,53 @@ def test_gather_combine(cuda):
     assert rel_err(out, (gathered * w[..., None]).sum(1)) < 1e-2
 
 
+@pytest.mark.parametrize("t,k,e,align", [(1, 1, 1, 128), (5, 3, 7, 128), (777, 4, 32, 128), (1000, 8, 128, 16), (300, 2, 1024, 1), (40000, 8, 128, 128)])
+def test_sorted_picks_match_the_plain_sort(cuda, t, k, e, align):
+    """Blocks, warps and steps of 32 picks, empty experts and one that takes most picks: the same
+    integers as the stable sort on the CPU."""
+    from bux_b200.ops import fused
+
+    torch.manual_seed(13)
+    picks = torch.randint(0, e, (t, k))
+    picks[torch.rand(t, k) < 0.5] = e // 2
+    w = torch.rand(t, k)
+    want = fused._sort_picks(picks, e, align, w)
+    got = fused._sort_picks(picks.cuda(), e, align, w.cuda())
+    for a, b in zip(got, want):
+        assert torch.equal(a.cpu(), b)
+
+
+def test_a_pick_of_no_expert_is_reported(cuda):
+    from bux_b200.ops import kernels as K
+
+    picks = torch.tensor([[0, 1], [1, 4], [-1, 0]], device=cuda)
+    row_index, pos, offsets, _ = K.sort_picks(picks, 4, 1, 6)
+    assert pos.tolist() == [[0, 2], [3, -2], [-2, 1]] and offsets.tolist() == [0, 2, 4, 4, 4]
+    assert row_index.tolist() == [0, 2, 0, 1, -1, -1]
+    out = K.combine_rows(torch.ones(6, 8, device=cuda).bfloat16(), pos, None, 3)
+    assert out[0].eq(2).all() and out[1:].isnan().all()
+    with pytest.raises(RuntimeError, match="2 waits"):
+        K.check_status(cuda)
+
+
+@pytest.mark.parametrize("rows,f", [(1, 8), (9, 248), (5, 264), (700, 768)])
+def test_glu_backward_rows(cuda, rows, f):
+    """One warp per row: rows narrower than a warp's step and remainders of it. Bounds: gradients
+    are rounded to bf16 (2^-9); the row scale's is an fp32 sum."""
+    from bux_b200.ops import kernels as K
+
+    torch.manual_seed(14)
+    h, dout = torch.randn(rows, 2 * f, device=cuda).bfloat16(), torch.randn(rows, f, device=cuda).bfloat16()
+    rs = torch.rand(rows, device=cuda)
+    hd, rd = h.double().requires_grad_(), rs.double().requires_grad_()
+    g, u = hd.clamp(max=1.5)[:, :f], hd.clamp(-1.5, 1.5)[:, f:]
+    (g * torch.sigmoid(g) * (u + 1) * rd[:, None]).backward(dout.double())
+    dh, drs = K.glu_bwd(h, dout, "swish", rs, 1.5, 1.0)
+    assert rel_err(dh, hd.grad) < 4e-3 and rel_err(drs, rd.grad) < 1e-4
+    into = torch.full((rows,), float("nan"), device=cuda)
+    assert torch.equal(K.glu_bwd_into(h, dout, "swish", rs, into, 1.5, 1.0), dh) and torch.equal(into, drs)
+
+
 @pytest.mark.parametrize("d,h,g", [(128, 4, 2), (64, 8, 2)])
 @pytest.mark.parametrize("t,window,sinks", [(256, 0, False), (300, 0, False), (384, 128, True)])
 def test_attention_fwd(cuda, d, h, g, t, window, sinks):
