@@ -632,20 +632,42 @@ glu_bwd_rows_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __
 //   sf_col tiles over (C, R_pad/32).
 constexpr int QT = 128;
 // The 128×128 bf16 tile sits in shared memory without padding, its 16-byte chunks (8 columns)
-// XOR-swizzled by the row, so that three access patterns are all free of bank conflicts:
-// eight consecutive chunks of a row (the load), one chunk of eight consecutive rows (the
-// row-wise pass) and one chunk of rows {8a + 2m + b} (the transposing ldmatrix of the column pass).
+// XOR-swizzled so that three access patterns are all free of bank conflicts: eight consecutive
+// chunks of a row (the load), chunk k of the four 32-column blocks of two adjacent rows (the
+// row-wise pass), and one chunk of the rows 32a + b, a < 4, b < 2 (the transposing ldmatrix of the
+// column pass).
 __device__ __forceinline__ int qtile_at(int row, int chunk) {
-  const int g = ((((row >> 3) ^ (row >> 1)) & 3) << 1) | (row & 1);
-  return row * QT + ((chunk ^ g) << 3);
+  const int g = (((row >> 5) & 3) << 1) | (row & 1);
+  return row * QT + (((chunk & 8) | ((chunk ^ g ^ ((chunk >> 3) << 1)) & 7)) << 3);
 }
-
+// The largest magnitude of 32 bf16 values in 16 words, two at a time (a NaN never wins).
+__device__ __forceinline__ float amax32(const uint32_t (&w)[16]) {
+  uint32_t m = w[0] & 0x7fff7fffu;
+#pragma unroll
+  for (int j = 1; j < 16; ++j) asm("max.bf16x2 %0, %1, %2;" : "=r"(m) : "r"(m), "r"(w[j] & 0x7fff7fffu));
+  const float2 t = unpack_bf16(m);
+  return fmaxf(t.x, t.y);
+}
+// 32 values times `inv` as e4m3 to 32 consecutive bytes: one 32-byte store where the address allows.
+__device__ __forceinline__ void store_e4m3x32(uint8_t* dst, const uint32_t (&w)[16], float inv, bool wide) {
+  uint32_t q[8];
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float2 a = unpack_bf16(w[2 * j]), b = unpack_bf16(w[2 * j + 1]);
+    q[j] = cvt_e4m3x4(a.x * inv, a.y * inv, b.x * inv, b.y * inv);
+  }
+  if (wide) {
+    asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(q[0]), "r"(q[1]), "r"(q[2]),
+                 "r"(q[3]), "r"(q[4]), "r"(q[5]), "r"(q[6]), "r"(q[7]) : "memory");
+  } else {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) reinterpret_cast<uint2*>(dst)[j] = make_uint2(q[2 * j], q[2 * j + 1]);
+  }
+}
 
 // What the quantiser reads its 128×128 tile from: the matrix itself, or a gated activation
 // computed on the way in (the activation, or its gradient, is then never written as bf16).
-#ifndef QUANT_CTAS
-#define QUANT_CTAS 5
-#endif
+constexpr int QUANT_CTAS = 5, QUANT_GLU_CTAS = 4;   // blocks per SM: 48 and 64 registers a thread
 enum { QSRC_PLAIN = 0, QSRC_GLU_FWD = 1, QSRC_GLU_BWD = 2, QSRC_MX = 3 };
 struct QuantGlu {
   const float* row_scale;     // PLAIN: output row r is its source row times row_scale[r] (rounded to bf16);
@@ -716,14 +738,17 @@ __device__ __forceinline__ uint4 glu_bwd8(const uint4& gv, const uint4& uv, cons
 }
 
 template <int SRC>
-__global__ void __launch_bounds__(256, QUANT_CTAS)
+__global__ void __launch_bounds__(256, SRC == QSRC_GLU_FWD || SRC == QSRC_GLU_BWD ? QUANT_GLU_CTAS : QUANT_CTAS)
 quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ x, long ld_x,
                    const int* __restrict__ row_index,
                    uint8_t* __restrict__ q_row, uint8_t* __restrict__ sf_row,
                    uint8_t* __restrict__ q_col, uint8_t* __restrict__ sf_col,
                    long rows, int cols, long ld_col, long x_batch_stride, QuantGlu gp) {
-  // Registers are kept low (values are re-read from the shared tile rather than held) so
-  // that six blocks fit an SM: the kernel is a stream, and blocks in flight hide its latency.
+  // What bounds it is the load / store unit: stores of 8 or 16 bytes per row of the output took a
+  // cycle each (65536 x 2048 both ways: 132 us at 75 % of its cycles, 24 instructions per element);
+  // with 32-byte stores and a whole block per thread 97 us (copying the bytes would take 83).
+  // outputs start on 32-byte boundaries (block offsets are multiples of 32)
+  const bool wide = ((reinterpret_cast<uintptr_t>(q_row) | reinterpret_cast<uintptr_t>(q_col)) & 31) == 0;
   __shared__ __align__(128) __nv_bfloat16 tile[QT * QT];
   __shared__ __align__(16) uint8_t sfr[512];
   __shared__ __align__(16) uint8_t sfc[512];
@@ -755,6 +780,25 @@ quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ x, long ld_x,
       }
       *reinterpret_cast<uint4*>(&tile[qtile_at(base * 16 + (tid >> 4), tid & 15)]) = v;
     }
+  } else if (SRC == QSRC_PLAIN && gp.row_scale == nullptr) {
+    // straight into the tile, all eight pieces of a thread in flight without registers; rows that
+    // do not exist are zeros. The gathered rows' numbers are read before the first copy is issued
+    // (between the copies each would wait for the one before:
+    // 139264 gathered rows of 2048 203 us, so 190).
+    long src[8];
+#pragma unroll
+    for (int base = 0; base < 8; ++base) {
+      const long r = r0 + base * 16 + (tid >> 4);
+      src[base] = r < rows ? (row_index ? (long)row_index[r] : r) : -1;
+    }
+#pragma unroll
+    for (int base = 0; base < 8; ++base) {
+      const bool live = src[base] >= 0 && c0 + cc < cols;
+      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&tile[qtile_at(base * 16 + (tid >> 4), tid & 15)]);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(live ? x + src[base] * ld_x + c0 + cc : x),
+                   "r"(live ? 16 : 0) : "memory");
+    }
+    asm volatile("cp.async.wait_all;" ::: "memory");
   } else if (SRC == QSRC_PLAIN) {
 #pragma unroll
     for (int base = 0; base < 8; base += 4) {
@@ -767,14 +811,12 @@ quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ x, long ld_x,
         v[i] = make_uint4(0, 0, 0, 0);
         if (r < rows && src >= 0 && c0 + cc < cols) {
           v[i] = *reinterpret_cast<const uint4*>(x + src * ld_x + c0 + cc);
-          if (gp.row_scale) {
-            const float rs = gp.row_scale[r];
-            uint32_t* u = &v[i].x;
+          const float rs = gp.row_scale[r];
+          uint32_t* u = &v[i].x;
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-              const float2 t = unpack_bf16(u[j]);
-              u[j] = pack_bf16(t.x * rs, t.y * rs);
-            }
+          for (int j = 0; j < 4; ++j) {
+            const float2 t = unpack_bf16(u[j]);
+            u[j] = pack_bf16(t.x * rs, t.y * rs);
           }
         }
       }
@@ -813,78 +855,50 @@ quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ x, long ld_x,
     }
   }
   __syncthreads();
+  // Both passes give a thread one whole 32-element block: its maximum needs no exchange, the scale is
+  // formed once, and it leaves as 32 bytes, four neighbours filling a 128-byte line.
+  const int lane = tid & 31, warp = tid >> 5;
   if (q_row) {
-    // thread -> row tid % 128, 32-column blocks tid / 128 and tid / 128 + 2
-    const int rr = tid & 127;
-    const long r = r0 + rr;
+    const int cb = lane & 3;
 #pragma unroll 1
     for (int i = 0; i < 2; ++i) {
-      const int cb = (tid >> 7) + 2 * i;
-      uint4 w[4];
-#pragma unroll
-      for (int k = 0; k < 4; ++k) w[k] = *reinterpret_cast<const uint4*>(&tile[qtile_at(rr, cb * 4 + k)]);
-      float amax = 0.f;
+      const int rr = i * 64 + warp * 8 + (lane >> 2);
+      const long r = r0 + rr;
+      uint32_t w[16];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const uint32_t* u = &w[k].x;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float2 t = unpack_bf16(u[j]);
-          amax = fmaxf(amax, fmaxf(fabsf(t.x), fabsf(t.y)));
-        }
+        const uint4 v = *reinterpret_cast<const uint4*>(&tile[qtile_at(rr, cb * 4 + k)]);
+        w[4 * k] = v.x; w[4 * k + 1] = v.y; w[4 * k + 2] = v.z; w[4 * k + 3] = v.w;
       }
       const bool live = r < rows && c0 + cb * 32 < cols;
-      const uint8_t e = e8m0_of(amax);
-      const float inv = e8m0_inv(e);
+      const uint8_t e = e8m0_of(amax32(w));
       sfr[(rr & 31) * 16 + (rr >> 5) * 4 + cb] = live ? e : (uint8_t)127;
-      if (live) {
-        uint4* dst = reinterpret_cast<uint4*>(q_row + r * cols + c0 + cb * 32);
-#pragma unroll
-        for (int hv = 0; hv < 2; ++hv) {
-          uint32_t packed[4];
-#pragma unroll
-          for (int k = 0; k < 2; ++k) {
-            const uint4& ww = w[2 * hv + k];
-            const float2 a = unpack_bf16(ww.x), b = unpack_bf16(ww.y), c = unpack_bf16(ww.z), d = unpack_bf16(ww.w);
-            packed[2 * k] = cvt_e4m3x4(a.x * inv, a.y * inv, b.x * inv, b.y * inv);
-            packed[2 * k + 1] = cvt_e4m3x4(c.x * inv, c.y * inv, d.x * inv, d.y * inv);
-          }
-          dst[hv] = make_uint4(packed[0], packed[1], packed[2], packed[3]);
-        }
-      }
+      if (live) store_e4m3x32(q_row + r * cols + c0 + cb * 32, w, e8m0_inv(e), wide);
     }
   }
   if (q_col) {
-    // A warp takes 8 columns × 32 rows at a time: one transposing ldmatrix hands each thread
-    // eight consecutive rows of one column (thread = column t/4, rows 8·(t%4)..+7), the four
-    // threads of a column share the block's maximum by two shuffles, and each writes 8 bytes.
-    const int warp = tid >> 5, lane = tid & 31;
+    // A warp takes 8 columns at a time. A transposing ldmatrix hands thread (column t / 4, q = t % 4)
+    // rows 2q and 2q + 1 of each 8x8 matrix; matrix m of load j holds the rows 32a + 8j + 2m + b, so
+    // after four loads of four the thread has rows 32q .. 32q + 31 of its column, in order.
     const int m = lane >> 3, i = lane & 7;  // this lane addresses row i of matrix m
     const int col = lane >> 2, q = lane & 3;
-#pragma unroll 2
-    for (int task = 0; task < 8; ++task) {
-      const int cg = warp * 2 + (task >> 2), rb = task & 3;
-      const int src_row = rb * 32 + 8 * (i >> 1) + 2 * m + (i & 1);
-      const uint32_t addr = (uint32_t)__cvta_generic_to_shared(&tile[qtile_at(src_row, cg)]);
-      uint32_t w0, w1, w2, w3;
-      asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
-                   : "=r"(w0), "=r"(w1), "=r"(w2), "=r"(w3) : "r"(addr));
-      const float2 a = unpack_bf16(w0), b = unpack_bf16(w1), c = unpack_bf16(w2), d = unpack_bf16(w3);
-      float amax = fmaxf(fmaxf(fmaxf(fabsf(a.x), fabsf(a.y)), fmaxf(fabsf(b.x), fabsf(b.y))),
-                         fmaxf(fmaxf(fabsf(c.x), fabsf(c.y)), fmaxf(fabsf(d.x), fabsf(d.y))));
-      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 1));
-      amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, 2));
+#pragma unroll 1
+    for (int task = 0; task < 2; ++task) {
+      const int cg = warp * 2 + task;
+      uint32_t w[16];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int src_row = 32 * (i >> 1) + 8 * j + 2 * m + (i & 1);
+        const uint32_t addr = (uint32_t)__cvta_generic_to_shared(&tile[qtile_at(src_row, cg)]);
+        asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+                     : "=r"(w[4 * j]), "=r"(w[4 * j + 1]), "=r"(w[4 * j + 2]), "=r"(w[4 * j + 3]) : "r"(addr));
+      }
       const int ccol = cg * 8 + col;
       const bool live = c0 + ccol < cols;
-      const uint8_t e = e8m0_of(amax);
-      const float inv = e8m0_inv(e);
-      if (q == 0) sfc[(ccol & 31) * 16 + (ccol >> 5) * 4 + rb] = live ? e : (uint8_t)127;
-      if (live) {
-        uint2 out;
-        out.x = cvt_e4m3x4(a.x * inv, a.y * inv, b.x * inv, b.y * inv);
-        out.y = cvt_e4m3x4(c.x * inv, c.y * inv, d.x * inv, d.y * inv);
-        *reinterpret_cast<uint2*>(q_col + (size_t)(c0 + ccol) * ld_col + r0 + rb * 32 + 8 * q) = out;
-      }
+      const uint8_t e = e8m0_of(amax32(w));
+      sfc[(ccol & 31) * 16 + (ccol >> 5) * 4 + q] = live ? e : (uint8_t)127;
+      if (live && r0 + 32 * q < ld_col)
+        store_e4m3x32(q_col + (size_t)(c0 + ccol) * ld_col + r0 + 32 * q, w, e8m0_inv(e), wide);
     }
   }
   __syncthreads();

@@ -56,6 +56,39 @@ def test_quant_mxfp8_matches_reference(cuda):
     assert torch.equal(q_col.view(torch.uint8), tq.view(torch.uint8))
 
 
+@pytest.mark.parametrize("rows,cols", [(1, 32), (31, 96), (129, 160), (300, 416)])
+@pytest.mark.parametrize("shift", [0, 8])
+def test_quant_mxfp8_ragged_gathered_and_shifted(cuda, rows, cols, shift):
+    """Partial tiles both ways, a row gather with absent rows, NaN and infinities, and outputs that do
+    not start on the 32-byte boundaries of the wide stores: the reference's bytes."""
+    from bux_b200.ops import kernels as K
+
+    torch.manual_seed(2)
+    src = torch.randn(40, cols, device=cuda).bfloat16()
+    src[3, 5], src[4, 7] = float("nan"), float("inf")
+    index = torch.randint(-1, 40, (rows,), device=cuda, dtype=torch.int32)
+    x = torch.where(index[:, None] >= 0, src[index.clamp_min(0).long()], torch.zeros(1, device=cuda, dtype=src.dtype))
+    r_pad = -(-rows // 128) * 128
+
+    def buffer(n):
+        return torch.empty(n + shift, dtype=torch.uint8, device=cuda)[shift:]
+
+    q_row, q_col = buffer(rows * cols), buffer(cols * r_pad)
+    # the scale tiles are whole 16-byte stores whatever the values' start
+    sf_row, sf_col = (torch.empty(K.sf_bytes(r, c), dtype=torch.uint8, device=cuda) for r, c in ((rows, cols), (cols, r_pad)))
+    K.ops().quant_mxfp8(src, index, None, q_row, sf_row, q_col, sf_col, rows, cols, r_pad, 1, 0)
+    xt = torch.zeros(cols, r_pad, device=cuda, dtype=torch.bfloat16)
+    xt[:, :rows] = x.t()
+    for got, sf, plain in ((q_row.view(rows, cols), sf_row, x), (q_col.view(cols, r_pad), sf_col, xt)):
+        finite = plain.isfinite().unflatten(-1, (-1, 32)).all(-1)
+        want, scales = ref.quant_mxfp8(plain.nan_to_num(0, 0, 0))
+        r, c = scales.shape
+        assert torch.equal(ref.unswizzle_scales(sf, r, c)[finite], scales[finite])
+        same = (got == want.view(torch.uint8)).unflatten(-1, (-1, 32)).all(-1)
+        assert same[finite].all()
+        assert (got.view(torch.float8_e4m3fn).float().isnan() == plain.isnan()).all()
+
+
 @pytest.mark.parametrize("m,n,k,bn", [(128, 128, 128, 128), (256, 384, 512, 128), (1000, 768, 2048, 128),
                                       (512, 512, 1024, 256)])
 def test_gemm_mxfp8(cuda, m, n, k, bn):
