@@ -648,13 +648,25 @@ __device__ __forceinline__ float amax32(const uint32_t (&w)[16]) {
   const float2 t = unpack_bf16(m);
   return fmaxf(t.x, t.y);
 }
+// 1 / 2^(e - 127) as bf16 (exact; e = 254 gives bf16's 2^-127).
+__device__ __forceinline__ unsigned short e8m0_inv_bf16(uint8_t e) {
+  return e < 254 ? (unsigned short)((254 - e) << 7) : (unsigned short)0x0040;
+}
+// Both values of a bf16 pair times a bf16 power of two, exactly, in fp32: one mixed-precision
+// multiply-add each (adding -0 keeps the sign of zeros) instead of a conversion and a product.
+__device__ __forceinline__ float2 scaled_bf16(uint32_t w, unsigned short inv) {
+  float2 t;
+  asm("fma.rn.f32.bf16 %0, %1, %2, %3;" : "=f"(t.x) : "h"((unsigned short)w), "h"(inv), "f"(-0.f));
+  asm("fma.rn.f32.bf16 %0, %1, %2, %3;" : "=f"(t.y) : "h"((unsigned short)(w >> 16)), "h"(inv), "f"(-0.f));
+  return t;
+}
 // 32 values times `inv` as e4m3 to 32 consecutive bytes: one 32-byte store where the address allows.
-__device__ __forceinline__ void store_e4m3x32(uint8_t* dst, const uint32_t (&w)[16], float inv, bool wide) {
+__device__ __forceinline__ void store_e4m3x32(uint8_t* dst, const uint32_t (&w)[16], unsigned short inv, bool wide) {
   uint32_t q[8];
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
-    const float2 a = unpack_bf16(w[2 * j]), b = unpack_bf16(w[2 * j + 1]);
-    q[j] = cvt_e4m3x4(a.x * inv, a.y * inv, b.x * inv, b.y * inv);
+    const float2 a = scaled_bf16(w[2 * j], inv), b = scaled_bf16(w[2 * j + 1], inv);
+    q[j] = cvt_e4m3x4(a.x, a.y, b.x, b.y);
   }
   if (wide) {
     asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(q[0]), "r"(q[1]), "r"(q[2]),
@@ -746,7 +758,7 @@ quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ x, long ld_x,
                    long rows, int cols, long ld_col, long x_batch_stride, QuantGlu gp) {
   // What bounds it is the load / store unit: stores of 8 or 16 bytes per row of the output took a
   // cycle each (65536 x 2048 both ways: 132 us at 75 % of its cycles, 24 instructions per element);
-  // with 32-byte stores and a whole block per thread 97 us (copying the bytes would take 83).
+  // with 32-byte stores and a whole block per thread 94 us (copying the bytes would take 83).
   // outputs start on 32-byte boundaries (block offsets are multiples of 32)
   const bool wide = ((reinterpret_cast<uintptr_t>(q_row) | reinterpret_cast<uintptr_t>(q_col)) & 31) == 0;
   __shared__ __align__(128) __nv_bfloat16 tile[QT * QT];
@@ -765,6 +777,9 @@ quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ x, long ld_x,
   const long r0 = (long)blockIdx.y * QT;
   const int c0 = blockIdx.x * QT;
   const int cc = (tid & 15) * 8;  // load: 16 threads per row (8 elements each), 16 rows per pass
+  // the place of this thread's piece of row 16 * base + tid / 16: bits 5-6 of the row are base / 2
+  const int place0 = qtile_at(tid >> 4, tid & 15);
+  auto place = [&](int base) { return (place0 ^ (((base >> 1) << 1) << 3)) + base * 16 * QT; };
   if (SRC == QSRC_MX) {
     // the source is already MXFP8 along its columns (what a peer pushed): dequantise into the
     // tile; the column pass below then quantises along the rows
@@ -778,13 +793,13 @@ quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ x, long ld_x,
         const uint2 q = *reinterpret_cast<const uint2*>(x8 + r * ld_x + c0 + cc);
         v = dequant_e4m3x8(q, gp.src_sf[sf_offset(r, (c0 + cc) >> 5, src_sf_cols)]);
       }
-      *reinterpret_cast<uint4*>(&tile[qtile_at(base * 16 + (tid >> 4), tid & 15)]) = v;
+      *reinterpret_cast<uint4*>(&tile[place(base)]) = v;
     }
   } else if (SRC == QSRC_PLAIN && gp.row_scale == nullptr) {
     // straight into the tile, all eight pieces of a thread in flight without registers; rows that
     // do not exist are zeros. The gathered rows' numbers are read before the first copy is issued
     // (between the copies each would wait for the one before:
-    // 139264 gathered rows of 2048 203 us, so 190).
+    // 139264 gathered rows of 2048 203 us, so 190; 173 since scaling takes one instruction).
     long src[8];
 #pragma unroll
     for (int base = 0; base < 8; ++base) {
@@ -794,7 +809,7 @@ quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ x, long ld_x,
 #pragma unroll
     for (int base = 0; base < 8; ++base) {
       const bool live = src[base] >= 0 && c0 + cc < cols;
-      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&tile[qtile_at(base * 16 + (tid >> 4), tid & 15)]);
+      const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&tile[place(base)]);
       asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(live ? x + src[base] * ld_x + c0 + cc : x),
                    "r"(live ? 16 : 0) : "memory");
     }
@@ -822,7 +837,7 @@ quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ x, long ld_x,
       }
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        *reinterpret_cast<uint4*>(&tile[qtile_at((base + i) * 16 + (tid >> 4), tid & 15)]) = v[i];
+        *reinterpret_cast<uint4*>(&tile[place(base + i)]) = v[i];
     }
   } else {
     // the tile is computed from h (and dout), two rows' loads in flight per thread.
@@ -850,7 +865,7 @@ quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ x, long ld_x,
         if (r < rows && c0 + cc < cols)
           o = SRC == QSRC_GLU_FWD ? glu_fwd8(g[i], u[i], gp, gp.row_scale ? gp.row_scale[r] : 1.f)
                                   : glu_bwd8(g[i], u[i], d[i], up_half, gp);
-        *reinterpret_cast<uint4*>(&tile[qtile_at((base + i) * 16 + (tid >> 4), tid & 15)]) = o;
+        *reinterpret_cast<uint4*>(&tile[place(base + i)]) = o;
       }
     }
   }
@@ -864,16 +879,18 @@ quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ x, long ld_x,
     for (int i = 0; i < 2; ++i) {
       const int rr = i * 64 + warp * 8 + (lane >> 2);
       const long r = r0 + rr;
+      // chunk cb * 4 + k differs from cb * 4 in its two low bits alone, and so does its place
+      const int first = qtile_at(rr, cb * 4);
       uint32_t w[16];
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
-        const uint4 v = *reinterpret_cast<const uint4*>(&tile[qtile_at(rr, cb * 4 + k)]);
+        const uint4 v = *reinterpret_cast<const uint4*>(&tile[first ^ (k << 3)]);
         w[4 * k] = v.x; w[4 * k + 1] = v.y; w[4 * k + 2] = v.z; w[4 * k + 3] = v.w;
       }
       const bool live = r < rows && c0 + cb * 32 < cols;
       const uint8_t e = e8m0_of(amax32(w));
       sfr[(rr & 31) * 16 + (rr >> 5) * 4 + cb] = live ? e : (uint8_t)127;
-      if (live) store_e4m3x32(q_row + r * cols + c0 + cb * 32, w, e8m0_inv(e), wide);
+      if (live) store_e4m3x32(q_row + r * cols + c0 + cb * 32, w, e8m0_inv_bf16(e), wide);
     }
   }
   if (q_col) {
@@ -885,11 +902,12 @@ quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ x, long ld_x,
 #pragma unroll 1
     for (int task = 0; task < 2; ++task) {
       const int cg = warp * 2 + task;
+      // the swizzle looks at bits 0 and 5-6 of the row: 8 rows further the chunk stays in its place
+      const uint32_t first = (uint32_t)__cvta_generic_to_shared(&tile[qtile_at(32 * (i >> 1) + 2 * m + (i & 1), cg)]);
       uint32_t w[16];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const int src_row = 32 * (i >> 1) + 8 * j + 2 * m + (i & 1);
-        const uint32_t addr = (uint32_t)__cvta_generic_to_shared(&tile[qtile_at(src_row, cg)]);
+        const uint32_t addr = first + j * 8 * QT * 2;
         asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
                      : "=r"(w[4 * j]), "=r"(w[4 * j + 1]), "=r"(w[4 * j + 2]), "=r"(w[4 * j + 3]) : "r"(addr));
       }
@@ -898,7 +916,7 @@ quant_mxfp8_kernel(const __nv_bfloat16* __restrict__ x, long ld_x,
       const uint8_t e = e8m0_of(amax32(w));
       sfc[(ccol & 31) * 16 + (ccol >> 5) * 4 + q] = live ? e : (uint8_t)127;
       if (live && r0 + 32 * q < ld_col)
-        store_e4m3x32(q_col + (size_t)(c0 + ccol) * ld_col + r0 + 32 * q, w, e8m0_inv(e), wide);
+        store_e4m3x32(q_col + (size_t)(c0 + ccol) * ld_col + r0 + 32 * q, w, e8m0_inv_bf16(e), wide);
     }
   }
   __syncthreads();
