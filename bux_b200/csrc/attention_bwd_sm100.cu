@@ -96,7 +96,7 @@ struct AttnBwdParams {
   const int* row_lo; const int* key_hi;  // documents: see AttnArgs
   float* dq; void* dk; void* dv; Status* status; unsigned int* phase_cycles;
   int B, T, S, H, G;
-  float scale, scale_log2; int causal, window;
+  float scale, scale_log2; int causal, window; bool by_length;
 };
 
 template <int D>
@@ -145,10 +145,12 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
   unsigned int* phase = reinterpret_cast<unsigned int*>(bars + B_COUNT + 1);   // 32 counters
 
   const int warp = threadIdx.x >> 5;
-  const int jt = blockIdx.x, g = blockIdx.y, b = blockIdx.z;
+  // key tile 0, which every query sees, first, over every head of a chunk
+  const AttnSlot slot = attn_slot(blockIdx.x, (p.S + BT - 1) / BT, p.G * p.B, p.by_length);
+  const int jt = slot.tile, g = slot.pair % p.G, b = slot.pair / p.G;
   // phase timers: one thread of softmax warp 0 and the MMA issuer of the first CTA add the
   // cycles since their last mark to a counter in shared memory
-  const bool timed = p.phase_cycles != nullptr && (blockIdx.x | blockIdx.y | blockIdx.z) == 0 &&
+  const bool timed = p.phase_cycles != nullptr && blockIdx.x == 0 &&
                      (threadIdx.x == 0 || warp == 9);
   unsigned int t_mark = timed ? (unsigned int)clock64() : 0u;
 #define BWD_MARK(slot)                                     \
@@ -496,7 +498,7 @@ attn_bwd_kernel(const __grid_constant__ AttnBwdParams p) {
 
   tc_fence_before();
   __syncthreads();
-  if (p.phase_cycles != nullptr && (blockIdx.x | blockIdx.y | blockIdx.z) == 0 && threadIdx.x < 32)
+  if (p.phase_cycles != nullptr && blockIdx.x == 0 && threadIdx.x < 32)
     atomicAdd(&p.phase_cycles[threadIdx.x], phase[threadIdx.x]);
   if (*abort_flag) {
     for (int i = 0; i < 64; ++i) __nanosleep(1000);
@@ -520,7 +522,7 @@ static const char* attn_bwd_launch_d(const AttnArgs& a, cudaStream_t stream) {
   p.lse = a.lse; p.delta = a.delta; p.dq = reinterpret_cast<float*>(a.dq); p.dk = a.dk; p.dv = a.dv;
   p.status = a.status; p.phase_cycles = a.phase_cycles;
   p.B = a.B; p.T = a.T; p.S = a.S; p.H = a.H; p.G = a.G;
-  p.scale = a.scale; p.scale_log2 = a.scale * LOG2E_B; p.causal = a.causal ? 1 : 0; p.window = a.window;
+  p.scale = a.scale; p.scale_log2 = a.scale * LOG2E_B; p.causal = a.causal ? 1 : 0; p.window = a.window; p.by_length = attn_by_length(a);
   auto kern = attn_bwd_kernel<D>;
   static bool configured[64] = {};
   if (!allow_dynamic_smem(kern, Cfg::SMEM_BYTES, configured))
@@ -528,8 +530,9 @@ static const char* attn_bwd_launch_d(const AttnArgs& a, cudaStream_t stream) {
   attn_delta_kernel<D><<<dim3((a.T + DELTA_T - 1) / DELTA_T, (a.H + DELTA_H - 1) / DELTA_H, a.B), 256, 0, stream>>>(
       reinterpret_cast<const __nv_bfloat16*>(a.o), reinterpret_cast<const __nv_bfloat16*>(a.d_o), a.lse,
       a.sinks, a.delta, a.dsinks, a.T, a.H, reinterpret_cast<uintptr_t>(a.o) % 16 == 0);
-  dim3 grid((a.S + BT - 1) / BT, a.G, a.B);
-  kern<<<grid, BWD_THREADS, Cfg::SMEM_BYTES, stream>>>(p);
+  const long grid = (long)((a.S + BT - 1) / BT) * a.G * a.B;
+  if (grid >= (1L << 31)) return "too many key tiles for one launch";
+  kern<<<(unsigned)grid, BWD_THREADS, Cfg::SMEM_BYTES, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? nullptr : "attention backward launch failed";
 }
 

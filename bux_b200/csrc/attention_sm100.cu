@@ -37,7 +37,7 @@ struct AttnFwdParams {
   void* o; float* lse; const float* sinks; Status* status;
   const int* row_lo;  // [B, T] first visible key of each query (documents), or null
   int B, T, S, H, G;
-  float scale_log2; int causal, window;
+  float scale_log2; int causal, window; bool by_length;
 };
 
 // Two 128-query tiles per CTA, one softmax warpgroup each, so that the tensor core
@@ -81,8 +81,10 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
 
   const int warp = threadIdx.x >> 5;
   const int n_qt = (p.T + 2 * QT - 1) / (2 * QT);
-  const int qt = n_qt - 1 - blockIdx.x;  // long (late) rows first under a causal mask
-  const int h = blockIdx.y, b = blockIdx.z;
+  // the longest (latest) rows first under a causal mask, over every head of a chunk
+  const AttnSlot slot = attn_slot(blockIdx.x, n_qt, p.H * p.B, p.by_length);
+  const int qt = n_qt - 1 - slot.tile;
+  const int h = slot.pair % p.H, b = slot.pair / p.H;
   const int g = h / (p.H / p.G);
   const int q0 = qt * 2 * QT;
   const int shift = p.S - p.T;
@@ -380,13 +382,14 @@ static const char* attn_fwd_launch_d(const AttnArgs& a, cudaStream_t stream) {
   p.o = a.o; p.lse = a.lse; p.sinks = a.sinks; p.status = a.status;
   p.row_lo = a.row_lo;
   p.B = a.B; p.T = a.T; p.S = a.S; p.H = a.H; p.G = a.G;
-  p.scale_log2 = a.scale * LOG2E; p.causal = a.causal ? 1 : 0; p.window = a.window;
+  p.scale_log2 = a.scale * LOG2E; p.causal = a.causal ? 1 : 0; p.window = a.window; p.by_length = attn_by_length(a);
   auto kern = attn_fwd_kernel<D>;
   static bool configured[64] = {};
   if (!allow_dynamic_smem(kern, Cfg::SMEM_BYTES, configured))
     return "cudaFuncSetAttribute(max dynamic shared memory) failed";
-  dim3 grid((a.T + 2 * QT - 1) / (2 * QT), a.H, a.B);
-  kern<<<grid, FWD_THREADS, Cfg::SMEM_BYTES, stream>>>(p);
+  const long grid = (long)((a.T + 2 * QT - 1) / (2 * QT)) * a.H * a.B;
+  if (grid >= (1L << 31)) return "too many query tiles for one launch";
+  kern<<<(unsigned)grid, FWD_THREADS, Cfg::SMEM_BYTES, stream>>>(p);
   return cudaGetLastError() == cudaSuccess ? nullptr : "attention forward launch failed";
 }
 
