@@ -404,6 +404,42 @@ def test_attention_fwd(cuda, d, h, g, t, window, sinks):
     assert rel_err(lse, want_lse) < 1e-3
 
 
+@pytest.mark.parametrize("t,s,causal,window,scale,spread", [
+    (1, 1, True, 0, None, 1.0),          # one query, one key
+    (127, 127, True, 0, None, 1.0),      # a tile that ends inside the row: no TMA store
+    (129, 300, True, 0, None, 1.0),      # more keys than queries; the second tile holds one row
+    (256, 191, False, 0, None, 1.0),     # no mask but the end of the keys, in a half tile
+    (300, 300, True, 40, None, 1.0),     # windows inside one half tile
+    (640, 640, True, 0, None, 40.0),     # scores of thousands: the rows' references move mid-way
+    (256, 256, True, 0, 0.0, 1.0),       # every score equal
+    (256, 256, True, 0, -0.1, 30.0),     # a negative scale
+])
+@pytest.mark.parametrize("d", [64, 128])
+def test_attention_fwd_edges(cuda, d, t, s, causal, window, scale, spread):
+    """Half tiles, partial tiles, references that move, against fp64. Bounds: P and the output are
+    rounded to bf16 (2^-9 each, against the largest probability)."""
+    from bux_b200.ops import kernels as K
+
+    torch.manual_seed(15)
+    q = torch.randn(2, t, 4, d, device=cuda).bfloat16()
+    k = (torch.randn(2, s, 2, d, device=cuda) * torch.linspace(0.1, spread, s, device=cuda)[None, :, None, None]).bfloat16()
+    v = torch.randn(2, s, 2, d, device=cuda).bfloat16()
+    sc = d ** -0.5 if scale is None else scale
+    z = torch.einsum("bthd,bshd->bhts", q.double(), k.double().repeat_interleave(2, 2)) * sc
+    i, j = torch.arange(t, device=cuda)[:, None] + s - t, torch.arange(s, device=cuda)[None]
+    hidden = (j > i) if causal else torch.zeros(t, s, dtype=torch.bool, device=cuda)
+    if window:
+        hidden = hidden | (j <= i - window)
+    z = z.masked_fill(hidden, float("-inf"))
+    want = torch.einsum("bhts,bshd->bthd", torch.softmax(z, -1).nan_to_num(0), v.double().repeat_interleave(2, 2))
+    got, lse = K.attn_fwd(q, k, v, causal=causal, window=window, scale=sc)
+    assert rel_err(got, want) < 6e-3
+    seen = ~hidden.all(-1)
+    ref_lse = torch.logsumexp(z, -1)
+    assert torch.allclose(lse.double()[..., seen], ref_lse[..., seen], rtol=1e-5, atol=1e-3)
+    assert (got[:, ~seen] == 0).all()
+
+
 @pytest.mark.parametrize("d,h,g", [(128, 4, 2), (64, 4, 1)])
 @pytest.mark.parametrize("t,window,sinks", [(256, 0, False), (300, 0, False), (384, 128, True)])
 def test_attention_bwd(cuda, d, h, g, t, window, sinks):
