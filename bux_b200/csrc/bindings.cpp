@@ -78,6 +78,17 @@ void gemm(const Tensor& a, const Tensor& b, Tensor& c, const c10::optional<Tenso
     g.wait_rows = (int)wait_rows; g.wait_on_k = wait_on_k; g.wait_on_n = wait_on_n;
   }
   g.m_rotate = (int)m_rotate;
+  Tensor partial;
+  if (g.bn == 0) {   // the tile width and a split of the contraction are chosen here
+    const bool may_split = g.mode == bux::MODE_DENSE && !wait_flags.has_value() && g.m_rotate == 0 &&
+                           (out_kind == bux::OUT_BF16 || out_kind == bux::OUT_F32);
+    const bux::GemmPlan plan = bux::gemm_plan(g.kind, M, N, K, g.sms, may_split);
+    g.bn = plan.bn;
+    if (plan.splits > 1) {
+      partial = at::empty({plan.splits, M, N}, c.options().dtype(at::kFloat));
+      g.splits = plan.splits; g.partial = partial.data_ptr<float>();
+    }
+  }
   const char* err = bux::gemm_launch(g, stream_of(a));
   TORCH_CHECK(err == nullptr, "bux gemm: ", err);
 }

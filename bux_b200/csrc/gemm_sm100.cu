@@ -61,7 +61,7 @@ struct GemmCfg {
 };
 
 struct TileCoord {
-  int group;    // expert index (0 when dense)
+  int group;    // expert index (dense: which range of the contraction)
   int m0;       // first row of A / C (global row in the sorted layout for MODE_GROUPED_ROWS)
   int m_end;    // one past the last valid row
   int n0;
@@ -85,15 +85,17 @@ struct TileWalk {
     if (p.mode == MODE_DENSE) {
       int m_tiles = (p.M + BM - 1) / BM;
       int total = m_tiles * n_tiles;
-      if (t >= total) return c;
+      if (t >= total * p.splits) return c;
+      const int split = t / total, tile = t % total;
       constexpr int GM = 16;
       int per_super = GM * n_tiles;
-      int sup = t / per_super, local = t % per_super;
+      int sup = tile / per_super, local = tile % per_super;
       int rows_here = min(GM, m_tiles - sup * GM);
       int mt = sup * GM + local % rows_here;
       int nt = local / rows_here;
       if (p.m_rotate) mt = (mt + p.m_rotate) % m_tiles;
-      c.group = 0; c.m0 = mt * BM; c.m_end = p.M; c.n0 = nt * bn; c.k0 = 0; c.k1 = p.K;
+      c.group = split; c.m0 = mt * BM; c.m_end = p.M; c.n0 = nt * bn;
+      c.k0 = split * p.k_split; c.k1 = min(p.K, c.k0 + p.k_split);
       c.valid = true;
     } else if (p.mode == MODE_GROUPED_ROWS) {
       while (g < p.groups) {
@@ -311,7 +313,7 @@ gemm_sm100_kernel(const __grid_constant__ GemmParams p) {
       const bool row_ok = row < c.m_end;
       const bool empty_k = c.k0 >= c.k1;
       size_t out_row = (size_t)row;
-      if (p.mode == MODE_GROUPED_K) out_row += (size_t)c.group * p.M;
+      if (p.mode != MODE_GROUPED_ROWS) out_row += (size_t)c.group * p.M;
       const uint32_t t_addr = tmem_base + acc * BN + ((uint32_t)(quad * 32) << 16);
       // full bf16 tiles leave through shared memory and TMA stores: whole 128-byte lines,
       // asynchronous, and the accumulator is released as soon as it has been read
@@ -320,7 +322,7 @@ gemm_sm100_kernel(const __grid_constant__ GemmParams p) {
       const bool out_adds = p.out_kind == OUT_F32_ACC || p.out_kind == OUT_BF16_ACC;
       if (by_tma) {
         uint8_t* mine = epi_smem + (warp - 2) * 4096;
-        const int out_row0 = (p.mode == MODE_GROUPED_K ? c.group * p.M : 0) + c.m0 + quad * 32;
+        const int out_row0 = (p.mode != MODE_GROUPED_ROWS ? c.group * p.M : 0) + c.m0 + quad * 32;
         // a slab is 32 rows x 128 bytes: 64 bf16 columns, or 32 fp32 columns
         const int slab_cols = out_bf16 ? 64 : 32;
 #pragma unroll 1
@@ -518,8 +520,95 @@ static const char* launch_cfg(const GemmParams& p, int sms, cudaStream_t stream)
   return cudaGetLastError() == cudaSuccess ? nullptr : "gemm kernel launch failed";
 }
 
-const char* gemm_launch(const GemmArgs& a, cudaStream_t stream) {
+// out[i] = sum over the ranges of part[r][i], in order; four elements per thread (N % 4 == 0), or one.
+template <typename OT, int V>
+__global__ void __launch_bounds__(256) sum_splits_kernel(const float* __restrict__ part, OT* __restrict__ out, long m, int n, long ldc, int splits) {
+  const long total = m * n / V, plane = m * n;
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (long)gridDim.x * blockDim.x) {
+    const long e = i * V, row = e / n;
+    float acc[V];
+#pragma unroll
+    for (int j = 0; j < V; ++j) acc[j] = 0.f;
+#pragma unroll 4
+    for (int s = 0; s < splits; ++s) {
+      if (V == 4) {
+        const float4 v = *reinterpret_cast<const float4*>(part + s * plane + e);
+        acc[0] += v.x; acc[1 % V] += v.y; acc[2 % V] += v.z; acc[3 % V] += v.w;
+      } else {
+        acc[0] += part[s * plane + e];
+      }
+    }
+    OT* dst = out + row * ldc + (e - row * n);
+#pragma unroll
+    for (int j = 0; j < V; ++j) dst[j] = (OT)acc[j];
+  }
+}
+
+// One wave of 256-wide tiles costs 1, of 128-wide ones 0.62 (more operand traffic per product: 8192^3
+// 0.54, 32768 x 5120 x 2048 0.62, 16384 x 14336 x 4096 0.65 of the wide tile's time), so the narrow tile is taken where it
+// saves enough of a last wave. Where even its tiles leave half of the SMs idle, the contraction is cut
+// as well, in ranges of at least four steps: a small product is a stream of its operands, and what
+// bounds it is how many SMs read. 16 x 6144 x 4096 (48 narrow tiles): 23.4 us with 24 wide tiles (29 with cold operands), 14.5 in 3
+// ranges and their sum.
+GemmPlan gemm_plan(int kind, long M, long N, long K, int sms, bool may_split) {
+  if (sms <= 0) sms = 148;
+  const long mt = (M + BM - 1) / BM, wide = mt * ((N + 255) / 256), narrow = mt * ((N + 127) / 128);
+  const bool wide_fits = kind == KIND_BF16 || N % 256 == 0;
+  GemmPlan plan{256, 1};
+  if (!wide_fits || (narrow + sms - 1) / sms * 0.62 < (double)((wide + sms - 1) / sms)) plan.bn = 128;
+  const long steps = (K + (kind == KIND_BF16 ? 63 : 127)) / (kind == KIND_BF16 ? 64 : 128);
+  if (may_split && plan.bn == 128 && narrow > 0 && narrow * 2 <= sms && steps >= 8)
+    plan.splits = (int)(sms / narrow < steps / 4 ? sms / narrow : steps / 4);
+  return plan;
+}
+
+static const char* launch_kernel(const GemmArgs& a, const GemmParams& p, int sms, cudaStream_t stream) {
+  const int bn = a.bn;
+#define BUX_GEMM_CASE(KIND_, BN_, AMN_, BMN_) \
+  if (a.kind == KIND_ && bn == BN_ && a.a_mn == AMN_ && a.b_mn == BMN_) \
+    return launch_cfg<KIND_, BN_, AMN_, BMN_>(p, sms, stream);
+  BUX_GEMM_CASE(KIND_BF16, 256, false, false)
+  BUX_GEMM_CASE(KIND_BF16, 256, false, true)
+  BUX_GEMM_CASE(KIND_BF16, 256, true, false)
+  BUX_GEMM_CASE(KIND_BF16, 256, true, true)
+  BUX_GEMM_CASE(KIND_BF16, 128, false, false)
+  BUX_GEMM_CASE(KIND_BF16, 128, false, true)
+  BUX_GEMM_CASE(KIND_BF16, 128, true, false)
+  BUX_GEMM_CASE(KIND_BF16, 128, true, true)
+  BUX_GEMM_CASE(KIND_MXFP8, 128, false, false)
+  if (a.kind == KIND_MXFP8 && bn == 256 && a.mode == MODE_GROUPED_ROWS)
+    return launch_cfg<KIND_MXFP8, 256, false, false, 8>(p, sms, stream);
+  BUX_GEMM_CASE(KIND_MXFP8, 256, false, false)
+#undef BUX_GEMM_CASE
+  return "no gemm kernel for this configuration";
+}
+
+
+static const char* sum_splits(const GemmArgs& a, cudaStream_t stream) {
+  const bool vec = a.N % 4 == 0;
+  const long threads = (long)a.M * a.N / (vec ? 4 : 1);
+  const int grid = (int)((threads + 255) / 256 < 148 * 8 ? (threads + 255) / 256 : 148 * 8);
+  if (a.out_kind == OUT_BF16) {
+    if (vec) sum_splits_kernel<__nv_bfloat16, 4><<<grid, 256, 0, stream>>>(a.partial, (__nv_bfloat16*)a.c, a.M, a.N, a.ldc, a.splits);
+    else sum_splits_kernel<__nv_bfloat16, 1><<<grid, 256, 0, stream>>>(a.partial, (__nv_bfloat16*)a.c, a.M, a.N, a.ldc, a.splits);
+  } else {
+    if (vec) sum_splits_kernel<float, 4><<<grid, 256, 0, stream>>>(a.partial, (float*)a.c, a.M, a.N, a.ldc, a.splits);
+    else sum_splits_kernel<float, 1><<<grid, 256, 0, stream>>>(a.partial, (float*)a.c, a.M, a.N, a.ldc, a.splits);
+  }
+  return cudaGetLastError() == cudaSuccess ? nullptr : "summing the ranges of a split product failed to launch";
+}
+
+const char* gemm_launch(const GemmArgs& args, cudaStream_t stream) {
+  GemmArgs a = args;
+  const bool split = a.splits > 1;
+  if (split) {
+    if (a.mode != MODE_DENSE || a.partial == nullptr || (a.out_kind != OUT_BF16 && a.out_kind != OUT_F32)) return "only a dense product that writes C can be split";
+    a.c = a.partial; a.ldc = a.N; a.out_kind = OUT_F32;
+  }
   GemmParams p;
+  p.splits = split ? a.splits : 1;
+  const int step = a.kind == KIND_BF16 ? 64 : 128;
+  p.k_split = ((a.K + step - 1) / step + p.splits - 1) / p.splits * step;
   p.mode = a.mode; p.M = a.M; p.N = a.N; p.K = a.K; p.k_total = a.k_total > 0 ? a.k_total : a.K;
   p.groups = a.groups; p.group_offsets = a.group_offsets;
   p.c = a.c; p.ldc = a.ldc; p.out_kind = a.out_kind;
@@ -543,32 +632,21 @@ const char* gemm_launch(const GemmArgs& a, cudaStream_t stream) {
   p.tma_store = 0;
   const int c_elem = (a.out_kind == OUT_BF16 || a.out_kind == OUT_BF16_ACC) ? 2 : 4;
   if (a.ldc * c_elem % 16 == 0 && reinterpret_cast<uintptr_t>(a.c) % 16 == 0 &&
-      (a.mode != MODE_GROUPED_K || a.M % BM == 0)) {
+      ((a.mode != MODE_GROUPED_K && !split) || a.M % BM == 0)) {
     // rows of C: every row the walk can touch (grouped rows: the sorted, padded row count;
     // grouped contraction: the groups' [M, N] outputs stacked). Boxes are 32 rows x 128 bytes;
     // fp32 accumulation into C is a TMA reduce-add (no read of C by the SMs).
-    const uint64_t rows = a.mode == MODE_GROUPED_K ? (uint64_t)a.groups * a.M : (uint64_t)a.M;
+    const uint64_t rows = a.mode == MODE_GROUPED_K ? (uint64_t)a.groups * a.M : (uint64_t)a.M * p.splits;
     if (make_tmap_2d(&p.tmap_c, a.c, c_elem, rows, (uint64_t)a.N, (uint64_t)a.ldc * c_elem, 128 / c_elem, 32) == nullptr)
       p.tma_store = 1;
   }
-  const int sms = a.sms > 0 ? a.sms : 148;
-#define BUX_GEMM_CASE(KIND_, BN_, AMN_, BMN_) \
-  if (a.kind == KIND_ && bn == BN_ && a.a_mn == AMN_ && a.b_mn == BMN_) \
-    return launch_cfg<KIND_, BN_, AMN_, BMN_>(p, sms, stream);
-  BUX_GEMM_CASE(KIND_BF16, 256, false, false)
-  BUX_GEMM_CASE(KIND_BF16, 256, false, true)
-  BUX_GEMM_CASE(KIND_BF16, 256, true, false)
-  BUX_GEMM_CASE(KIND_BF16, 256, true, true)
-  BUX_GEMM_CASE(KIND_BF16, 128, false, false)
-  BUX_GEMM_CASE(KIND_BF16, 128, false, true)
-  BUX_GEMM_CASE(KIND_BF16, 128, true, false)
-  BUX_GEMM_CASE(KIND_BF16, 128, true, true)
-  BUX_GEMM_CASE(KIND_MXFP8, 128, false, false)
-  if (a.kind == KIND_MXFP8 && bn == 256 && a.mode == MODE_GROUPED_ROWS)
-    return launch_cfg<KIND_MXFP8, 256, false, false, 8>(p, sms, stream);
-  BUX_GEMM_CASE(KIND_MXFP8, 256, false, false)
-#undef BUX_GEMM_CASE
-  return "no gemm kernel for this configuration";
+  int sms = a.sms > 0 ? a.sms : 148;
+  if (a.mode == MODE_DENSE) {   // no block without a tile
+    const long tiles = (long)((a.M + BM - 1) / BM) * ((a.N + bn - 1) / bn) * p.splits;
+    if (tiles < sms) sms = tiles > 0 ? (int)tiles : 1;
+  }
+  err = launch_kernel(a, p, sms, stream);
+  if (err == nullptr && split) err = sum_splits(args, stream);
+  return err;
 }
-
 }  // namespace bux

@@ -28,6 +28,7 @@ struct GemmParams {
   const int* wait_flags; int wait_world, wait_epoch; unsigned long long wait_limit_ns;
   // wait_rows > 0: per-sender row blocks (see GemmArgs); m_rotate in tiles
   int wait_rows, m_rotate, wait_on_k, wait_on_n;
+  int splits, k_split;  // dense: the contraction in `splits` ranges of k_split, each into its own [M, N] of C
   int tma_store;  // the epilogue stages bf16 tiles in shared memory and stores them by TMA
 };
 
@@ -51,8 +52,15 @@ struct GemmArgs {
   // the sender of its rows. m_rotate (dense mode, in tiles) starts the walk at this
   // rank's own rows, which need no wait.
   int wait_rows = 0, m_rotate = 0; bool wait_on_k = false;
+  // dense, bf16 or fp32 output: the contraction in this many ranges, each into its own fp32 [M, N] of
+  // `partial`, summed into C by a second kernel
+  int splits = 1; float* partial = nullptr;
   bool wait_on_n = false;  // the senders write row blocks of B (sharded weights arriving from their owners)
 };
+
+// Tile width and number of contraction ranges for a dense product, from how full the SMs get.
+struct GemmPlan { int bn, splits; };
+GemmPlan gemm_plan(int kind, long M, long N, long K, int sms, bool may_split);
 
 // Returns nullptr on success, else a static message.
 const char* gemm_launch(const GemmArgs& args, cudaStream_t stream);

@@ -274,11 +274,11 @@ class _LinearF32Out(torch.autograd.Function):
         if w.dtype == torch.float32:
             hi = w.to(torch.bfloat16)
             lo = (w - hi.float()).to(torch.bfloat16)
-            y2 = K.gemm_bf16(x2, torch.cat((hi, lo), dim=0), out_dtype=torch.float32, bn=256 if 2 * n > 128 else 128)
+            y2 = K.gemm_bf16(x2, torch.cat((hi, lo), dim=0), out_dtype=torch.float32)
             y = y2[:, :n] + y2[:, n:]
             wb = hi
         else:
-            y = K.gemm_bf16(x2, w, out_dtype=torch.float32, bn=128 if n <= 128 else 256)
+            y = K.gemm_bf16(x2, w, out_dtype=torch.float32)
             wb = w
         ctx.save_for_backward(x2, wb)
         ctx.shape, ctx.w_dtype = x.shape, w.dtype

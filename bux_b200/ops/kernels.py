@@ -60,9 +60,10 @@ def check_status(device, what: str = "kernel") -> None:
 # ------------------------------------------------------------------ GEMM
 def gemm_bf16(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: bool = False,
               out: Optional[torch.Tensor] = None, out_dtype=torch.bfloat16,
-              accumulate: bool = False, bn: int = 256, sms: int = 0, wait_flags=None, wait_epoch: int = 0,
+              accumulate: bool = False, bn: int = 0, sms: int = 0, wait_flags=None, wait_epoch: int = 0,
               wait_rows: int = 0, m_rotate: int = 0, wait_on_k: bool = False, wait_on_n: bool = False) -> torch.Tensor:
-    """C = A · B^T. A is [M,K] (or stored [K,M] with a_mn), B is [N,K] (or [K,N] with b_mn).
+    """C = A · B^T, `bn` columns per tile (0: chosen by size, and the contraction split where the
+    product is too small to fill the SMs). A is [M,K] (or stored [K,M] with a_mn), B is [N,K] (or [K,N] with b_mn).
     With `wait_flags` (int32[senders]) an operand is being written by peer GPUs in blocks
     of `wait_rows` rows per sender (rows of A, of the contraction with `wait_on_k`, or rows of B
     with `wait_on_n`: a weight whose shards arrive from their owners):
@@ -87,7 +88,7 @@ def _tile_width(n: int) -> int:
 def gemm_mxfp8(aq, asf, bq, bsf, m: int, n: int, k: int, *, out=None, out_dtype=torch.bfloat16,
                accumulate: bool = False, bn: Optional[int] = None, sms: int = 0) -> torch.Tensor:
     """C[m,n] = dequant(A)[m,k] · dequant(B)[n,k]^T; scales in the tiled layout."""
-    bn = _tile_width(n) if bn is None else bn
+    bn = 0 if bn is None else bn
     if out is None:
         out = _out(m, n, dtype=out_dtype, device=aq.device, op="gemm_mxfp8")
     kind = OUT_BF16 if out.dtype == torch.bfloat16 else (OUT_F32_ACC if accumulate else OUT_F32)

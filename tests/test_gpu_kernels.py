@@ -205,6 +205,37 @@ def test_norm_rope_odd_heads(cuda, tokens, heads, d):
     assert rel_err(y, want) < 4e-3 and rel_err(dx, xr.grad) < 4e-3 and rel_err(dw, wr.grad) < 1e-5
 
 
+@pytest.mark.parametrize("m,n,k", [(1, 8, 512), (16, 6144, 4096), (130, 136, 1000), (128, 256, 2048), (3, 2048, 568), (509, 1024, 3072)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_small_products_are_split(cuda, m, n, k, a_mn, b_mn, dtype):
+    """Products too small to fill the SMs: one row, ragged edges of the tiles and of the last range of
+    the contraction. Bounds: bf16 outputs are rounded once (2^-9); in fp32 the tensor core cuts its
+    accumulator's low bits once per 16 terms, 2^-23 of it each time (measured 1.4e-6 at k = 4096)."""
+    from bux_b200.ops import kernels as K
+
+    if a_mn and m % 8:
+        pytest.skip("an MN-major operand's rows are whole 16-byte pieces")
+    torch.manual_seed(16)
+    a, b = torch.randn(m, k, device=cuda).bfloat16(), torch.randn(n, k, device=cuda).bfloat16()
+    want = a.double() @ b.double().t()
+    out = K.gemm_bf16(a.t().contiguous() if a_mn else a, b.t().contiguous() if b_mn else b, a_mn=a_mn, b_mn=b_mn, out_dtype=dtype)
+    assert rel_err(out, want) < (4e-3 if dtype == torch.bfloat16 else k / 16 * 2 ** -23)
+    again = K.gemm_bf16(a.t().contiguous() if a_mn else a, b.t().contiguous() if b_mn else b, a_mn=a_mn, b_mn=b_mn, out_dtype=dtype)
+    assert torch.equal(out, again)
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 128, 1024), (100, 384, 2048), (128, 256, 4096)])
+def test_small_mxfp8_products_are_split(cuda, m, n, k):
+    from bux_b200.ops import kernels as K
+
+    torch.manual_seed(17)
+    aq, asf, _, _ = K.quant_mxfp8(torch.randn(m, k, device=cuda).bfloat16())
+    bq, bsf, _, _ = K.quant_mxfp8(torch.randn(n, k, device=cuda).bfloat16())
+    wide = [ref.dequant_mxfp8(q, ref.unswizzle_scales(sf, q.shape[0], k // 32)).double() for q, sf in ((aq, asf), (bq, bsf))]
+    assert rel_err(K.gemm_mxfp8(aq, asf, bq, bsf, m, n, k), wide[0] @ wide[1].t()) < 4e-3
+
+
 @pytest.mark.parametrize("d", [64, 128])
 @pytest.mark.parametrize("norm", [True, False])
 def test_norm_rope(cuda, d, norm):
