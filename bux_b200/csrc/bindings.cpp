@@ -7,12 +7,13 @@
 #include <torch/library.h>
 
 #include "attention_sm100.h"
+#include "bindings.h"
 #include "comm_sm100.h"
 #include "elementwise.h"
 #include "gemm_sm100.h"
 #include "scan_sm100.h"
 
-namespace {
+namespace bux_ops {
 
 using at::Tensor;
 
@@ -529,9 +530,10 @@ void ep_wait(const Tensor& flags, int64_t epoch, const c10::optional<Tensor>& st
   bux::ep_wait(flags.data_ptr<int>(), (int)flags.numel(), (int)epoch, (uint64_t)(limit_s * 1e9), status_ptr(status), stream_of(flags));
 }
 
-}  // namespace
+}  // namespace bux_ops
 
 TORCH_LIBRARY(bux_b200, m) {
+  using namespace bux_ops;
   m.def("ep_push_rows(Tensor x, Tensor src_token, Tensor dst_rank, Tensor dst_row, Tensor? row_scale, Tensor peer_base, int sms, Tensor? peer_scale=None) -> ()", &ep_push_rows);
   m.def("ep_push_rows_mx(Tensor x, Tensor rank_of, Tensor row_of, Tensor? w, Tensor peer_q, Tensor peer_sf, Tensor? peer_scale, int sms) -> ()", &ep_push_rows_mx);
   m.def("requant_mxfp8_cols(Tensor q, Tensor sf, Tensor(a!) q_col, Tensor(b!) sf_col, int rows, int cols, int ld_col) -> ()", &requant_mxfp8_cols);

@@ -15,6 +15,7 @@ from typing import Optional
 import torch
 import torch.nn.functional as F
 
+from . import checks
 from . import reference as ref
 
 _OFF = os.environ.get("BUX_KERNELS", "").lower() == "off"
@@ -33,6 +34,20 @@ def _K():
     from . import kernels
 
     return kernels
+
+
+_ad: dict = {}
+
+
+def _native(name: str):
+    """The C++ autograd function `name` (csrc/autograd.cpp); None with kernel checks on, which put every
+    output between guards and so take the Python functions below."""
+    if checks.enabled():
+        return None
+    op = _ad.get(name)
+    if op is None:
+        op = _ad[name] = getattr(_K().ops(), name).default
+    return op
 
 
 # ------------------------------------------------------------------ norms
@@ -58,7 +73,8 @@ def rmsnorm(x, weight, eps: float = 1e-6, zero_centered: bool = False):
         w = weight
         if zero_centered and w is not None:
             w = w + 1.0
-        return _RMSNorm.apply(x, w, eps)
+        native = _native("ad_rmsnorm")
+        return _RMSNorm.apply(x, w, eps) if native is None else native(x, w, eps)
     return ref.rmsnorm(x, weight, eps, zero_centered)
 
 
@@ -87,6 +103,9 @@ def rmsnorm_rope(x, weight, cos, sin, eps: float = 1e-6):
     x: [B, T, H, D]; cos/sin: [B, T, D/2] fp32."""
     d = x.shape[-1]
     if kernels_on(x) and d in (64, 128, 256) and cos.shape[-1] * 2 == d:
+        native = _native("ad_norm_rope")
+        if native is not None:
+            return native(x, weight, cos, sin, eps)
         c2 = cos.reshape(-1, d // 2).float().contiguous()
         s2 = sin.reshape(-1, d // 2).float().contiguous()
         return _NormRope.apply(x, weight, c2, s2, eps)
@@ -127,6 +146,9 @@ def glu(h, kind: str = "swish", row_scale=None, limit: Optional[float] = None,
     f = h.shape[-1] // 2
     K_ok = kernels_on(h) and f % 8 == 0 and kind in ("swish", "quick_gelu", "gelu_tanh", "relu2")
     if K_ok:
+        native = _native("ad_glu")
+        if native is not None:
+            return native(h, row_scale, _K().ACT_KINDS[kind], float(limit or 0.0), float(up_offset))
         return _GLU.apply(h, row_scale, kind, float(limit or 0.0), float(up_offset))
     out = ref.glu(h[..., :f], h[..., f:], kind, limit, up_offset)
     if row_scale is not None:
@@ -326,7 +348,9 @@ def linear(x, w, bias=None, fmt: str = "bf16", passes=PASSES):
         if fmt in ("mxfp8", "mxfp8_2d") and k % 128 == 0 and n % 128 == 0:
             y = _LinearMX.apply(x, w, passes)
         else:
-            y = _LinearBF16.apply(x, w, getattr(w, "_bux_arrival", None))
+            arrival = getattr(w, "_bux_arrival", None)
+            native = _native("ad_linear") if arrival is None and getattr(w, "main_grad", None) is None else None
+            y = _LinearBF16.apply(x, w, arrival) if native is None else native(x, w, _K().status_word(x.device))
         return y if bias is None else y + bias.to(y.dtype)
     if fmt in ("mxfp8", "mxfp8_2d") and k % 32 == 0 and not x.is_cuda and "fprop" in passes:
         return ref_linear_mxfp8(x, w, bias)
@@ -431,7 +455,13 @@ def attention(q, k, v, *, causal: bool = True, window: Optional[int] = None, sin
     native = (kernels_on(q) and d in (64, 128) and v.shape[-1] == d and softcap is None
               and (not packed or (causal and q.shape[1] == k.shape[1] and torch.is_tensor(segments))))
     if native:
-        return _Attention.apply(q, k, v, sinks, causal, int(window or 0), scale, segments)
+        op = _native("ad_attention") if attention_replay is None else None
+        if op is None:
+            return _Attention.apply(q, k, v, sinks, causal, int(window or 0), scale, segments)
+        K = _K()
+        row_lo, key_hi = K.document_bounds(segments) if packed else (None, None)
+        return op(q, k, v, sinks, row_lo, key_hi, K.status_word(q.device), causal, int(window or 0),
+                  float(scale if scale is not None else d ** -0.5))
     if (q.is_cuda and softcap is None and segments is None and sinks is None and window is None
             and q.dtype in (torch.bfloat16, torch.float16)):
         # library baseline (BUX_KERNELS=off, or a head dim the kernel does not take)

@@ -18,7 +18,7 @@ OUT_BF16, OUT_F32, OUT_F32_ACC, OUT_BF16_ACC = 0, 1, 2, 3
 ACT_KINDS = {"swish": 0, "quick_gelu": 1, "gelu_tanh": 2, "relu2": 3}
 
 _status: dict = {}
-launches = 0  # kernels launched through this module (bench.py reports it)
+_launches = 0  # kernels launched through this module
 
 
 def ops():
@@ -34,8 +34,16 @@ def _out(*shape, dtype, device, op: str, fill=None) -> torch.Tensor:
 
 
 def _count(n: int = 1) -> None:
-    global launches
-    launches += n
+    global _launches
+    _launches += n
+
+
+def __getattr__(name: str):
+    """``launches``: the library's kernels launched so far, through this module and by the C++ autograd
+    functions (bench.py reports it)."""
+    if name == "launches":
+        return _launches + (ops().native_launches() if _build._loaded else 0)
+    raise AttributeError(f"module {__name__!r} has no attribute {name!r}")
 
 
 def status_word(device) -> torch.Tensor:

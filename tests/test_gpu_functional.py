@@ -234,3 +234,93 @@ methods = methods(microbatches=4, remat=full{more})
     assert out["plain"][0] == pytest.approx(out["interleaved"][0], abs=1e-3)
     for name, p in out["plain"][1].items():
         assert rel_err(out["interleaved"][1][name], p) < 1e-3, name
+
+
+def _layer_calls(cuda):
+    """One call of each layer op on inputs that are odd on purpose: slices, transposes, other dtypes."""
+    from bux_b200 import ops
+
+    g = torch.Generator(device=cuda).manual_seed(3)
+
+    def rand(*shape, dtype=torch.bfloat16):
+        return torch.randn(*shape, generator=g, device=cuda).to(dtype)
+
+    qkv = rand(2, 40, 3 * 4 * 64)
+    cos, sin = torch.rand(2, 40, 32, device=cuda).double(), torch.rand(2, 40, 32, device=cuda)
+    seg = torch.tensor([[0] * 15 + [1] * 25, [0] * 40], device=cuda)
+    return {
+        "rmsnorm": ([rand(520, 6).t(), rand(520)], lambda x, w: ops.rmsnorm(x, w, 1e-5)),
+        "rmsnorm plain": ([rand(2, 3, 64)], lambda x: ops.rmsnorm(x, None)),
+        "rmsnorm zero-centred": ([rand(2, 3, 64), rand(64, dtype=torch.float32)], lambda x, w: ops.rmsnorm(x, w, 1e-6, True)),
+        "norm + rope of a slice": ([qkv, rand(64)], lambda x, w: ops.rmsnorm_rope(x[..., 256:512].unflatten(-1, (4, 64)), w, cos, sin)),
+        "rope": ([rand(2, 4, 40, 64)], lambda x: ops.rope(x.transpose(1, 2), cos, sin)),
+        "glu": ([rand(2, 9, 48)], lambda h: ops.glu(h, "gelu_tanh", None, 7.0, 1.0)),
+        "glu scaled": ([rand(9, 48), rand(9)], lambda h, s: ops.glu(h, "swish", s)),
+        "linear": ([rand(2, 24, 9), rand(40, 24)], lambda x, w: ops.linear(x.transpose(1, 2), w)),
+        "linear with bias": ([rand(3, 24), rand(40, 24), rand(40)], ops.linear),
+        "attention": ([rand(2, 40, 4, 64), rand(2, 40, 2, 64), rand(2, 2, 40, 64)],
+                      lambda q, k, v: ops.attention(q, k, v.transpose(1, 2), window=16)),
+        "attention packed": ([rand(2, 40, 4, 64), rand(2, 40, 2, 64), rand(2, 40, 2, 64), rand(4)],
+                             lambda q, k, v, s: ops.attention(q, k, v, sinks=s, segments=seg, scale=0.2)),
+    }
+
+
+@pytest.mark.parametrize("frozen", [None, 0, 1])
+def test_native_autograd_functions_match_the_python_ones(cuda, frozen, monkeypatch):
+    """The same kernels, casts and saved tensors: outputs, gradients, their dtypes and strides, launch
+    counts; with any one input frozen, under saved-tensor hooks, without gradients. Bits, but for what
+    the kernels themselves sum with atomics (dq, the gains of the rotation, the sinks)."""
+    from bux_b200.ops import functional as F
+    from bux_b200.ops import kernels as K
+
+    def packed(x):
+        return x.cpu()
+
+    def run(name, inputs, fn, hooks):
+        xs = [x.detach().clone().requires_grad_(i != frozen) for i, x in enumerate(inputs)]
+        before = K.launches
+        with torch.autograd.graph.saved_tensors_hooks(packed, lambda x: x.to(cuda)) if hooks else torch.enable_grad():
+            y = fn(*xs)
+        want = [x for x in xs if x.requires_grad]
+        grads = torch.autograd.grad(y, want, torch.ones_like(y) * 0.1, allow_unused=True) if want else []
+        with torch.no_grad():
+            again = fn(*xs)
+        assert torch.equal(again, y) and not again.requires_grad
+        return [y, *grads], K.launches - before
+
+    for name, (inputs, fn) in _layer_calls(cuda).items():
+        for hooks in (False, True):
+            got, n = run(name, inputs, fn, hooks)
+            with monkeypatch.context() as m:
+                m.setattr(F, "_native", lambda op: None)
+                want, n_want = run(name, inputs, fn, hooks)
+            assert n == n_want, name
+            for a, b in zip(got, want):
+                assert a.dtype == b.dtype and a.shape == b.shape and a.stride() == b.stride(), name
+                assert torch.equal(a, b) or torch.allclose(a.float(), b.float(), rtol=2 ** -7, atol=1e-5), name
+
+
+def test_native_autograd_functions_refuse_and_recompute(cuda):
+    """Forward-mode differentiation stays refused; a checkpointed call recomputes; gradients of
+    gradients are not made up."""
+    from torch.utils.checkpoint import checkpoint
+
+    from bux_b200 import ops
+
+    x = torch.randn(4, 64, device=cuda).bfloat16().requires_grad_()
+    w = torch.randn(64, device=cuda).requires_grad_()
+    plain = torch.autograd.grad(ops.rmsnorm(x, w).sum(), [x, w])
+    for reentrant in (True, False):
+        y = checkpoint(lambda a, b: ops.rmsnorm(a, b), x, w, use_reentrant=reentrant)
+        if reentrant:
+            x.grad = w.grad = None
+            y.sum().backward()
+            again = [x.grad, w.grad]
+        else:
+            again = torch.autograd.grad(y.sum(), [x, w])
+        assert all(torch.equal(a, b) for a, b in zip(plain, again))
+    dx, = torch.autograd.grad(ops.rmsnorm(x, w).sum(), [x], create_graph=True)
+    assert not dx.requires_grad or dx.grad_fn is not None
+    with pytest.raises((NotImplementedError, RuntimeError)):
+        with torch.autograd.forward_ad.dual_level():
+            ops.rmsnorm(torch.autograd.forward_ad.make_dual(x.detach(), torch.ones_like(x)), w)
