@@ -124,6 +124,40 @@ struct TileWalk {
   }
 };
 
+// One row of an epilogue slab (128 bytes, TMA's 128-byte swizzle) from tensor memory: 64 columns as
+// bf16 or 32 as fp32.
+__device__ __forceinline__ void epilogue_slab(uint8_t* rowp, uint32_t t_addr, int lane, bool out_bf16, bool zero) {
+  if (out_bf16) {
+    uint32_t r0[32], r1[32];
+    tmem_ld_x32(t_addr, r0);
+    tmem_ld_x32(t_addr + 32, r1);
+    tmem_ld_wait();
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {
+      const uint32_t* src = v < 4 ? &r0[8 * v] : &r1[8 * (v - 4)];
+      uint4 q;
+      if (zero) {
+        q = make_uint4(0, 0, 0, 0);
+      } else {
+        q.x = pack_bf16(__uint_as_float(src[0]), __uint_as_float(src[1]));
+        q.y = pack_bf16(__uint_as_float(src[2]), __uint_as_float(src[3]));
+        q.z = pack_bf16(__uint_as_float(src[4]), __uint_as_float(src[5]));
+        q.w = pack_bf16(__uint_as_float(src[6]), __uint_as_float(src[7]));
+      }
+      *reinterpret_cast<uint4*>(rowp + ((v ^ (lane & 7)) << 4)) = q;
+    }
+  } else {
+    uint32_t r0[32];
+    tmem_ld_x32(t_addr, r0);
+    tmem_ld_wait();
+#pragma unroll
+    for (int v = 0; v < 8; ++v) {
+      uint4 q = zero ? make_uint4(0, 0, 0, 0) : make_uint4(r0[4 * v], r0[4 * v + 1], r0[4 * v + 2], r0[4 * v + 3]);
+      *reinterpret_cast<uint4*>(rowp + ((v ^ (lane & 7)) << 4)) = q;
+    }
+  }
+}
+
 template <int KIND, int BN, bool A_MN, bool B_MN, int EW = 4>
 __global__ void __launch_bounds__((GemmCfg<KIND, BN, EW>::THREADS), 1)
 gemm_sm100_kernel(const __grid_constant__ GemmParams p) {
@@ -336,37 +370,7 @@ gemm_sm100_kernel(const __grid_constant__ GemmParams p) {
             else tma_store_wait_read();
           }
           __syncwarp();
-          uint8_t* rowp = slab + lane * 128;
-          if (out_bf16) {
-            uint32_t r0[32], r1[32];
-            tmem_ld_x32(t_addr + col, r0);
-            tmem_ld_x32(t_addr + col + 32, r1);
-            tmem_ld_wait();
-#pragma unroll
-            for (int v = 0; v < 8; ++v) {
-              const uint32_t* src = v < 4 ? &r0[8 * v] : &r1[8 * (v - 4)];
-              uint4 q;
-              if (empty_k) {
-                q = make_uint4(0, 0, 0, 0);
-              } else {
-                q.x = pack_bf16(__uint_as_float(src[0]), __uint_as_float(src[1]));
-                q.y = pack_bf16(__uint_as_float(src[2]), __uint_as_float(src[3]));
-                q.z = pack_bf16(__uint_as_float(src[4]), __uint_as_float(src[5]));
-                q.w = pack_bf16(__uint_as_float(src[6]), __uint_as_float(src[7]));
-              }
-              *reinterpret_cast<uint4*>(rowp + ((v ^ (lane & 7)) << 4)) = q;
-            }
-          } else {
-            uint32_t r0[32];
-            tmem_ld_x32(t_addr + col, r0);
-            tmem_ld_wait();
-#pragma unroll
-            for (int v = 0; v < 8; ++v) {
-              uint4 q = empty_k ? make_uint4(0, 0, 0, 0)
-                                : make_uint4(r0[4 * v], r0[4 * v + 1], r0[4 * v + 2], r0[4 * v + 3]);
-              *reinterpret_cast<uint4*>(rowp + ((v ^ (lane & 7)) << 4)) = q;
-            }
-          }
+          epilogue_slab(slab + lane * 128, t_addr + col, lane, out_bf16, empty_k);
           fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) {
@@ -459,6 +463,179 @@ gemm_sm100_kernel(const __grid_constant__ GemmParams p) {
     tc_fence_after();
     tmem_dealloc(tmem_base, Cfg::TMEM_COLS);
   }
+}
+
+// ------------------------------------------------------------------ pairs of SMs
+// The dense bf16 product on CTA pairs: one 256 x 256 tile per pair, each CTA holding 128 rows of A and
+// 128 columns of B. Each operand byte then enters shared memory once per 256 x 256 products instead of
+// once per 128 x 256, a third less traffic: what a product under the power cap is paid in, since the tensor
+// cores' rate follows the clock that is left. Back to back, single CTAs and pairs: 8192 x 14336 x 4096
+// 1279 and 1342 TFLOP/s, 4096 x 151936 x 2048 1226 and 1315, its gradients 1173 and 1226, 1256 and 1331.
+// Roles as above; both producers fill their own shared memory and count on rank 0's barrier, rank 0
+// issues the MMAs, and their completion arrives in both CTAs.
+struct PairCfg {
+  static constexpr int BN = 256, HALF = 128, BK = 64;
+  static constexpr int A_BYTES = 128 * 128, B_BYTES = 128 * 128, STAGE_BYTES = A_BYTES + B_BYTES;
+  static constexpr int STAGES = 6, ACC_STAGES = 2, EPI_WARPS = 4;
+  static constexpr int EPI_BYTES = 2 * EPI_WARPS * 4096;
+  static constexpr int THREADS = 64 + 32 * EPI_WARPS;
+  static constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + EPI_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+};
+constexpr int KID_GEMM_PAIR = 7;
+
+template <bool A_MN, bool B_MN>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PairCfg::THREADS, 1)
+gemm_pair_kernel(const __grid_constant__ GemmParams p) {
+  using Cfg = PairCfg;
+  constexpr int STAGES = Cfg::STAGES;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  uint8_t* epi_smem = smem + STAGES * Cfg::STAGE_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(epi_smem + Cfg::EPI_BYTES);
+  uint64_t* full = bars;                       // used in rank 0: bytes of both CTAs
+  uint64_t* empty = bars + STAGES;             // in each CTA: the pair's MMAs have read the stage
+  uint64_t* acc_full = bars + 2 * STAGES;      // in each CTA
+  uint64_t* acc_empty = acc_full + Cfg::ACC_STAGES;  // used in rank 0: both CTAs' epilogue warps
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + Cfg::ACC_STAGES);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = cluster_rank();
+  Status* st = p.status;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+    for (int a = 0; a < Cfg::ACC_STAGES; ++a) { mbar_init(&acc_full[a], 1); mbar_init(&acc_empty[a], 2 * Cfg::EPI_WARPS); }
+    *abort_flag = 0;
+    mbar_fence_init();
+  }
+  if (warp == 1) { tmem_alloc_pair(tmem_slot, 512); tmem_relinquish_pair(); }
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();   // the other CTA's barriers are ready, and so is its tensor memory
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  const int m_tiles = (p.M + 255) / 256, n_tiles = (p.N + 255) / 256, total = m_tiles * n_tiles;
+  const int pairs = gridDim.x >> 1;
+  // super-rows of 8 tiles, as many rows of A as the single-CTA walk keeps in L2
+  auto tile_at = [&](int t, int& m0, int& n0) {
+    constexpr int GM = 8;
+    const int sup = t / (GM * n_tiles), local = t % (GM * n_tiles), rows_here = min(GM, m_tiles - sup * GM);
+    m0 = (sup * GM + local % rows_here) * 256 + (int)rank * 128;
+    n0 = local / rows_here * 256;
+  };
+  if (warp == 0) {
+    // ------------------------------------------------------------ TMA producer (both CTAs)
+    if (elect_one()) {
+      tma_prefetch_desc(&p.tmap_a);
+      tma_prefetch_desc(&p.tmap_b);
+      int stage = 0; uint32_t phase = 0;
+      bool ok = true;
+      for (int t = blockIdx.x >> 1; t < total && ok; t += pairs) {
+        int m0, n0;
+        tile_at(t, m0, n0);
+        const int nb = n0 + (int)rank * Cfg::HALF;
+        for (int k = 0; k < p.K; k += Cfg::BK) {
+          ok = mbar_wait(&empty[stage], phase ^ 1, abort_flag, st, KID_GEMM_PAIR, 1);
+          if (!ok) break;
+          uint8_t* sa = smem + stage * Cfg::STAGE_BYTES;
+          uint8_t* sb = sa + Cfg::A_BYTES;
+          // the pair's bytes of a stage, expected once; the other CTA's may arrive before this
+          if (rank == 0) mbar_expect_tx(&full[stage], 2 * Cfg::STAGE_BYTES);
+          const uint32_t bar = cluster_addr(&full[stage], 0);
+          if (A_MN) {
+            for (int j = 0; j < 2; ++j) tma_load_2d_pair(sa + j * (Cfg::BK * 128), &p.tmap_a, m0 + j * 64, k, bar);
+          } else {
+            tma_load_2d_pair(sa, &p.tmap_a, k, m0, bar);
+          }
+          if (B_MN) {
+            for (int j = 0; j < 2; ++j) tma_load_2d_pair(sb + j * (Cfg::BK * 128), &p.tmap_b, nb + j * 64, k, bar);
+          } else {
+            tma_load_2d_pair(sb, &p.tmap_b, k, nb, bar);
+          }
+          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------ MMA issuer (rank 0)
+    if (rank == 0 && elect_one()) {
+      constexpr uint32_t idesc = make_idesc(FMT_BF16, FMT_BF16, 256, 256, A_MN, B_MN);
+      int stage = 0; uint32_t phase = 0;
+      int acc = 0; uint32_t acc_phase = 0;
+      bool ok = true;
+      for (int t = blockIdx.x >> 1; t < total && ok; t += pairs) {
+        ok = mbar_wait<true>(&acc_empty[acc], acc_phase ^ 1, abort_flag, st, KID_GEMM_PAIR, 2);
+        if (!ok) break;
+        tc_fence_after();
+        const uint32_t d_tmem = tmem_base + acc * Cfg::BN;
+        uint32_t accumulate = 0;
+        for (int k = 0; k < p.K; k += Cfg::BK) {
+          ok = mbar_wait<true>(&full[stage], phase, abort_flag, st, KID_GEMM_PAIR, 3);
+          if (!ok) break;
+          tc_fence_after();
+          const uint32_t sa = smem_u32(smem + stage * Cfg::STAGE_BYTES), sb = sa + Cfg::A_BYTES;
+#pragma unroll
+          for (int kk = 0; kk < Cfg::BK / 16; ++kk) {
+            const uint64_t ad = A_MN ? make_smem_desc(sa + kk * 2048, Cfg::BK * 128, 1024, 2) : make_smem_desc(sa + kk * 32, 0, 1024, 2);
+            const uint64_t bd = B_MN ? make_smem_desc(sb + kk * 2048, Cfg::BK * 128, 1024, 2) : make_smem_desc(sb + kk * 32, 0, 1024, 2);
+            mma_f16_pair(d_tmem, ad, bd, idesc, accumulate);
+            accumulate = 1;
+          }
+          tc_commit_pair(&empty[stage]);
+          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+        }
+        if (!ok) break;
+        tc_commit_pair(&acc_full[acc]);
+        if (++acc == Cfg::ACC_STAGES) { acc = 0; acc_phase ^= 1; }
+      }
+    }
+  } else {
+    // ------------------------------------------------------------ epilogue (both CTAs, their own 128 rows)
+    const int quad = warp & 3;
+    int acc = 0; uint32_t acc_phase = 0;
+    int epi_round = 0;
+    bool ok = true;
+    const bool out_bf16 = p.out_kind == OUT_BF16 || p.out_kind == OUT_BF16_ACC;
+    const bool out_adds = p.out_kind == OUT_F32_ACC || p.out_kind == OUT_BF16_ACC;
+    for (int t = blockIdx.x >> 1; t < total && ok; t += pairs) {
+      ok = warp_all(mbar_wait(&acc_full[acc], acc_phase, abort_flag, st, KID_GEMM_PAIR, 4));
+      if (!ok) break;
+      tc_fence_after();
+      int m0, n0;
+      tile_at(t, m0, n0);
+      const uint32_t t_addr = tmem_base + acc * Cfg::BN + ((uint32_t)(quad * 32) << 16);
+      const bool rows_here = m0 + quad * 32 < p.M;   // stores do not start past the last row
+#pragma unroll 1
+      for (int col = 0; col < Cfg::BN && rows_here; col += out_bf16 ? 64 : 32) {
+        if (n0 + col >= p.N) break;
+        uint8_t* slab = epi_smem + (warp - 2) * 4096 + (epi_round & 1) * (Cfg::EPI_WARPS * 4096);
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");   // the store before last has read it
+        __syncwarp();
+        epilogue_slab(slab + lane * 128, t_addr + col, lane, out_bf16, false);
+        fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          if (out_adds) tma_reduce_add_2d(&p.tmap_c, slab, n0 + col, m0 + quad * 32);
+          else tma_store_2d(&p.tmap_c, slab, n0 + col, m0 + quad * 32);
+          tma_store_commit();
+        }
+        ++epi_round;
+      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(cluster_addr(&acc_empty[acc], 0));
+      if (++acc == Cfg::ACC_STAGES) { acc = 0; acc_phase ^= 1; }
+    }
+  }
+  if (warp >= 2 && lane == 0) tma_store_wait_all();
+  tc_fence_before();
+  __syncthreads();
+  if (*abort_flag) {
+    for (int i = 0; i < 64; ++i) __nanosleep(1000);
+    __syncthreads();
+  }
+  cluster_sync();   // neither CTA leaves while the other's loads, MMAs or arrivals may still reach it
+  if (warp == 1) { tc_fence_after(); tmem_dealloc_pair(tmem_base, 512); }
 }
 
 // ------------------------------------------------------------------ host side
@@ -584,6 +761,33 @@ static const char* launch_kernel(const GemmArgs& a, const GemmParams& p, int sms
 }
 
 
+// Pairs take the dense bf16 products of wide tiles that fill them: at least a wave of 256 x 256 tiles
+// (with fewer neither is better: 64 tiles of 2048 x 2048 x 4096 30 us both, 20 of 512 x 4096 x 4096 25 and 27),
+// C where TMA can store it, nothing arriving from other GPUs.
+constexpr int PAIR_MIN_TILES = 74;
+static bool takes_pairs(const GemmArgs& a) {
+  const long tiles = (long)((a.M + 255) / 256) * ((a.N + 255) / 256);
+  const int c_elem = (a.out_kind == OUT_BF16 || a.out_kind == OUT_BF16_ACC) ? 2 : 4;
+  return a.kind == KIND_BF16 && a.mode == MODE_DENSE && a.bn == 256 && a.splits <= 1 && a.wait_flags == nullptr &&
+         a.m_rotate == 0 && a.sms <= 0 && a.K > 0 && tiles >= PAIR_MIN_TILES && a.ldc * c_elem % 16 == 0 &&
+         reinterpret_cast<uintptr_t>(a.c) % 16 == 0;
+}
+
+template <bool A_MN, bool B_MN>
+static const char* launch_pair_as(const GemmParams& p, int ctas, cudaStream_t stream) {
+  auto kern = gemm_pair_kernel<A_MN, B_MN>;
+  static bool configured[64] = {};
+  if (!allow_dynamic_smem(kern, PairCfg::SMEM_BYTES, configured)) return "cudaFuncSetAttribute(max dynamic shared memory) failed";
+  kern<<<ctas, PairCfg::THREADS, PairCfg::SMEM_BYTES, stream>>>(p);
+  return cudaGetLastError() == cudaSuccess ? nullptr : "gemm kernel launch failed";
+}
+static const char* launch_pair(const GemmArgs& a, const GemmParams& p, cudaStream_t stream) {
+  const long tiles = (long)((a.M + 255) / 256) * ((a.N + 255) / 256);
+  const int ctas = tiles < 74 ? 2 * (int)tiles : 148;
+  if (a.a_mn) return a.b_mn ? launch_pair_as<true, true>(p, ctas, stream) : launch_pair_as<true, false>(p, ctas, stream);
+  return a.b_mn ? launch_pair_as<false, true>(p, ctas, stream) : launch_pair_as<false, false>(p, ctas, stream);
+}
+
 static const char* sum_splits(const GemmArgs& a, cudaStream_t stream) {
   const bool vec = a.N % 4 == 0;
   const long threads = (long)a.M * a.N / (vec ? 4 : 1);
@@ -619,6 +823,7 @@ const char* gemm_launch(const GemmArgs& args, cudaStream_t stream) {
   const int elem = a.kind == KIND_BF16 ? 2 : 1;
   const int bk = a.kind == KIND_BF16 ? 64 : 128;
   const int bn = a.bn;
+  const bool pair = takes_pairs(a);
   if (a.kind == KIND_MXFP8 && (a.a_mn || a.b_mn)) return "mxfp8 operands are K-major";
   if (a.kind == KIND_MXFP8 && (p.k_total % 128 != 0)) return "mxfp8 K must be a multiple of 128";
   const char* err;
@@ -627,7 +832,7 @@ const char* gemm_launch(const GemmArgs& args, cudaStream_t stream) {
   else        err = make_tmap_2d(&p.tmap_a, a.a, elem, a.a_outer, a.a_inner, a.lda_bytes, bk, BM);
   if (err) return err;
   if (a.b_mn) err = make_tmap_2d(&p.tmap_b, a.b, elem, a.b_outer, a.b_inner, a.ldb_bytes, 64, bk);
-  else        err = make_tmap_2d(&p.tmap_b, a.b, elem, a.b_outer, a.b_inner, a.ldb_bytes, bk, bn);
+  else        err = make_tmap_2d(&p.tmap_b, a.b, elem, a.b_outer, a.b_inner, a.ldb_bytes, bk, pair ? 128 : bn);
   if (err) return err;
   p.tma_store = 0;
   const int c_elem = (a.out_kind == OUT_BF16 || a.out_kind == OUT_BF16_ACC) ? 2 : 4;
@@ -639,6 +844,10 @@ const char* gemm_launch(const GemmArgs& args, cudaStream_t stream) {
     const uint64_t rows = a.mode == MODE_GROUPED_K ? (uint64_t)a.groups * a.M : (uint64_t)a.M * p.splits;
     if (make_tmap_2d(&p.tmap_c, a.c, c_elem, rows, (uint64_t)a.N, (uint64_t)a.ldc * c_elem, 128 / c_elem, 32) == nullptr)
       p.tma_store = 1;
+  }
+  if (pair) {
+    if (!p.tma_store) return "a product on CTA pairs stores by TMA";
+    return launch_pair(a, p, stream);
   }
   int sms = a.sms > 0 ? a.sms : 148;
   if (a.mode == MODE_DENSE) {   // no block without a tile

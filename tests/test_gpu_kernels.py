@@ -225,6 +225,23 @@ def test_small_products_are_split(cuda, m, n, k, a_mn, b_mn, dtype):
     assert torch.equal(out, again)
 
 
+@pytest.mark.parametrize("m,n,k", [(2568, 2056, 200), (4224, 1288, 64), (8, 18952, 72), (2048, 2560, 1024)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
+@pytest.mark.parametrize("out", ["bf16", "f32", "f32 +="])
+def test_products_on_pairs_of_sms(cuda, m, n, k, a_mn, b_mn, out):
+    """Enough 256 x 256 tiles for CTA pairs: tiles of which one CTA's rows or columns lie outside, one
+    step and ragged steps of the contraction, all layouts, stores and additions. Bounds as above."""
+    from bux_b200.ops import kernels as K
+
+    torch.manual_seed(18)
+    a, b = torch.randn(m, k, device=cuda).bfloat16(), torch.randn(n, k, device=cuda).bfloat16()
+    want = a.double() @ b.double().t()
+    into = torch.ones(m, n, device=cuda) if out == "f32 +=" else None
+    got = K.gemm_bf16(a.t().contiguous() if a_mn else a, b.t().contiguous() if b_mn else b, a_mn=a_mn, b_mn=b_mn, bn=256, out=into,
+                      out_dtype=torch.bfloat16 if out == "bf16" else torch.float32, accumulate=into is not None)
+    assert rel_err(got, want + 1 if into is not None else want) < (4e-3 if out == "bf16" else 3e-6)
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 128, 1024), (100, 384, 2048), (128, 256, 4096)])
 def test_small_mxfp8_products_are_split(cuda, m, n, k):
     from bux_b200.ops import kernels as K
