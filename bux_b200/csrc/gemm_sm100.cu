@@ -362,7 +362,8 @@ gemm_sm100_kernel(const __grid_constant__ GemmParams p) {
 #pragma unroll 1
         for (int col = col_begin; col < col_begin + EPI_COLS; col += slab_cols) {
           const int n = c.n0 + col;
-          if (n >= p.N) break;
+          // a warp's 32 rows lie in C's [M, N] of this group (range) or all outside, in the next one's
+          if (n >= p.N || c.m0 + quad * 32 >= c.m_end) break;
           uint8_t* slab = mine + (Cfg::EPI_SLABS == 2 ? (epi_round & 1) * (Cfg::EPI_WARPS * 4096) : 0);
           // the store that last read this slab must have finished reading it
           if (lane == 0) {
@@ -837,10 +838,12 @@ const char* gemm_launch(const GemmArgs& args, cudaStream_t stream) {
   p.tma_store = 0;
   const int c_elem = (a.out_kind == OUT_BF16 || a.out_kind == OUT_BF16_ACC) ? 2 : 4;
   if (a.ldc * c_elem % 16 == 0 && reinterpret_cast<uintptr_t>(a.c) % 16 == 0 &&
-      ((a.mode != MODE_GROUPED_K && !split) || a.M % BM == 0)) {
+      ((a.mode != MODE_GROUPED_K && !split) || a.M % 32 == 0)) {
     // rows of C: every row the walk can touch (grouped rows: the sorted, padded row count;
     // grouped contraction: the groups' [M, N] outputs stacked). Boxes are 32 rows x 128 bytes;
-    // fp32 accumulation into C is a TMA reduce-add (no read of C by the SMs).
+    // fp32 accumulation into C is a TMA reduce-add (no read of C by the SMs). Outputs stacked per group
+    // (per range) need whole boxes: M % 32 == 0 (32 x 2880 x 2880 with 128 rows each 225 us by rows from
+    // registers, as M % 128 != 0 took them before, 124 by TMA).
     const uint64_t rows = a.mode == MODE_GROUPED_K ? (uint64_t)a.groups * a.M : (uint64_t)a.M * p.splits;
     if (make_tmap_2d(&p.tmap_c, a.c, c_elem, rows, (uint64_t)a.N, (uint64_t)a.ldc * c_elem, 128 / c_elem, 32) == nullptr)
       p.tma_store = 1;

@@ -88,9 +88,12 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: boo
     return out
 
 
-def _tile_width(n: int) -> int:
-    """256-wide tiles halve the operand traffic per FLOP; taken when they tile N exactly."""
-    return 256 if n % 256 == 0 else 128
+def _tile_width(n: int, kind: int) -> int:
+    """256-wide tiles halve the operand traffic per FLOP: taken when they tile N exactly, and in bf16
+    (whose operands need no whole scale tiles) where they cover at most a quarter more columns than
+    narrow ones (32 experts of 5760 x 2880, 128 rows each: 233 us wide, 282 narrow, 4 % more columns)."""
+    wide, narrow = -(-n // 256) * 256, -(-n // 128) * 128
+    return 256 if n % 256 == 0 or (kind == KIND_BF16 and wide * 4 <= narrow * 5) else 128
 
 
 def gemm_mxfp8(aq, asf, bq, bsf, m: int, n: int, k: int, *, out=None, out_dtype=torch.bfloat16,
@@ -111,7 +114,7 @@ def grouped_gemm(a, b, offsets: torch.Tensor, n: int, k: int, *, kind: int = KIN
                  wait_flags=None, wait_epoch: int = 0) -> torch.Tensor:
     """Rows of `a` ([R,k], sorted by group; offsets int32[G+1]) times group g's weight.
     b: [G*n, k] (K-major) or [G*k, n] (b_mn). Returns [R, n] bf16."""
-    bn = _tile_width(n) if bn is None else bn
+    bn = _tile_width(n, kind) if bn is None else bn
     groups = offsets.numel() - 1
     if out is None:
         out = _out(a.shape[0], n, dtype=torch.bfloat16, device=a.device, op="grouped_gemm")
@@ -131,7 +134,7 @@ def grouped_gemm_k(a, b, offsets: torch.Tensor, m: int, n: int, *, kind: int = K
     gradients of grouped experts). K-major: a [m, Ktot], b [n, Ktot]; MN-major: a [Ktot, m],
     b [Ktot, n]. Returns [G, m, n] in `out_dtype` (fp32, or bf16 written straight from the
     accumulator when that is what the gradient is kept in)."""
-    bn = _tile_width(n) if bn is None else bn
+    bn = _tile_width(n, kind) if bn is None else bn
     groups = offsets.numel() - 1
     ktot = a.shape[0] if a_mn else a.shape[1]
     if out is None:

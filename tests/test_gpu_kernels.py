@@ -149,6 +149,25 @@ def test_grouped_gemm_contraction(cuda):
     assert first[1].abs().max() == 0   # the empty group stays zero
 
 
+@pytest.mark.parametrize("m,n", [(32, 8), (160, 264), (224, 648), (72, 96)])
+@pytest.mark.parametrize("dtype,accumulate", [(torch.bfloat16, False), (torch.float32, False), (torch.float32, True)])
+def test_grouped_contraction_with_ragged_outputs(cuda, m, n, dtype, accumulate):
+    """Stacked outputs whose rows do not fill the tiles: whole 32-row boxes, and rows that are none (72).
+    Each group's gradient stays in its own rows. Bounds as for the dense products."""
+    from bux_b200.ops import kernels as K
+
+    torch.manual_seed(20)
+    offsets = torch.tensor([0, 128, 128, 320], dtype=torch.int32, device=cuda)
+    a, b = torch.randn(320, m, device=cuda).bfloat16(), torch.randn(320, n, device=cuda).bfloat16()
+    want = torch.stack([a[:128].double().t() @ b[:128].double(), torch.zeros(m, n, device=cuda, dtype=torch.float64),
+                        a[128:].double().t() @ b[128:].double()])
+    out = torch.ones(3, m, n, device=cuda, dtype=dtype) if accumulate else None
+    got = K.grouped_gemm_k(a, b, offsets, m, n, a_mn=True, b_mn=True, out=out, accumulate=accumulate, out_dtype=dtype)
+    for g in range(3):
+        assert rel_err(got[g], want[g] + int(accumulate)) < (4e-3 if dtype == torch.bfloat16 else 1e-6)
+    assert accumulate or (got[1] == 0).all()
+
+
 def test_rmsnorm(cuda):
     from bux_b200.ops import kernels as K
 
