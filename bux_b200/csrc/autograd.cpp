@@ -54,20 +54,16 @@ struct RMSNorm : torch::autograd::Function<RMSNorm> {
 };
 
 // ------------------------------------------------------------------ norm + RoPE
-// Elements between tokens of x [..., T, H, D] when heads are dense and the leading dimensions collapse
-// into one (a column slice of a fused projection); -1 otherwise (as `kernels.token_stride`).
-int64_t token_stride(const Tensor& x) {
-  const int64_t n = x.dim();
-  if (n < 3 || x.stride(-1) != 1 || x.stride(-2) != x.size(-1)) return -1;
-  const int64_t step = x.stride(-3);
-  for (int64_t i = n - 4; i >= 0; --i)
-    if (x.stride(i) != x.size(i + 1) * x.stride(i + 1)) return -1;
-  return step % 8 == 0 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 ? step : -1;
+// x as the kernel walks it: itself where it can be read in place (a column slice of a fused projection),
+// else a copy. `contiguous()` is no test of that: it returns x itself whatever the strides of its
+// dimensions of size 1 are, and wherever x starts.
+Tensor walkable(const Tensor& x) {
+  return token_stride(x) >= 0 ? x : x.clone(at::MemoryFormat::Contiguous);
 }
 
 struct NormRope : torch::autograd::Function<NormRope> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const OptTensor& w, const Tensor& cos, const Tensor& sin, double eps) {
-    const Tensor xc = token_stride(x) >= 0 ? x : x.contiguous();   // a slice of qkv is read in place
+    const Tensor xc = walkable(x);
     const int64_t d = xc.size(-1), h = xc.size(-2), tokens = xc.numel() / (h * d);
     const Tensor c = cos.reshape({-1, d / 2}).to(at::kFloat).contiguous(), s = sin.reshape({-1, d / 2}).to(at::kFloat).contiguous();
     const OptTensor wf = f32(w);
@@ -85,9 +81,8 @@ struct NormRope : torch::autograd::Function<NormRope> {
     const int64_t d = x.size(-1), h = x.size(-2), tokens = x.numel() / (h * d);
     Tensor dx = at::empty(x.sizes(), x.options()), dw;
     if (w.defined()) dw = at::zeros({d}, x.options().dtype(at::kFloat));
-    // a hook on saved tensors may have given x back with other strides
-    const Tensor xc = token_stride(x) >= 0 ? x : x.contiguous();
-    norm_rope(true, xc, f32(opt(w)), c, s, dx, opt(rstd), g[0].contiguous(), opt(dw), tokens, h, d, token_stride(xc), h * d,
+    const Tensor xc = walkable(x);   // a hook on saved tensors may have given x back with other strides
+    norm_rope(true, xc, f32(opt(w)), c, s, dx, opt(rstd), walkable(g[0].contiguous()), opt(dw), tokens, h, d, token_stride(xc), h * d,
               ctx->saved_data["eps"].toDouble());
     launched += 1;
     return {dx, w.defined() ? dw.to(w.scalar_type()) : Tensor(), Tensor(), Tensor(), Tensor()};

@@ -117,12 +117,36 @@ void rmsnorm_bwd(const Tensor& x, const c10::optional<Tensor>& w, const Tensor& 
   bux::rmsnorm_bwd(x.data_ptr(), opt_f32(w), dy.data_ptr(), rstd.data_ptr<float>(), dx.data_ptr(), dwp,
                    part.defined() ? part.data_ptr<float>() : nullptr, x.numel() / d, d, stream_of(x));
 }
-// x viewed as [tokens, heads, D] with token stride stride_x (elements); y likewise.
+int64_t token_stride(const Tensor& x) {
+  const int64_t n = x.dim();
+  if (n < 3) return -1;
+  const int64_t d = x.size(-1), h = x.size(-2);
+  if ((d > 1 && x.stride(-1) != 1) || (h > 1 && x.stride(-2) != d)) return -1;
+  // from the last dimension of more than one entry outwards; a dimension of one has no stride to agree with
+  int64_t step = -1, count = 1;
+  for (int64_t i = n - 3; i >= 0; --i) {
+    if (x.size(i) == 1) continue;
+    if (step < 0) step = x.stride(i);
+    else if (x.stride(i) != count * step) return -1;
+    count *= x.size(i);
+  }
+  if (step < 0) step = h * d;   // one token
+  return step >= h * d && step % 8 == 0 && reinterpret_cast<uintptr_t>(x.data_ptr()) % 16 == 0 ? step : -1;
+}
+// x viewed as [tokens, heads, D] with token stride stride_x (elements); y and dy are dense.
 void norm_rope(bool bwd, const Tensor& x, const c10::optional<Tensor>& w, const Tensor& cos, const Tensor& sin,
                Tensor& y, const c10::optional<Tensor>& rstd, const c10::optional<Tensor>& dy,
                const c10::optional<Tensor>& dw, int64_t tokens, int64_t heads, int64_t D,
                int64_t stride_x, int64_t stride_y, double eps) {
-  TORCH_CHECK(x.is_cuda() && y.is_cuda() && x.scalar_type() == at::kBFloat16, "norm_rope: bf16 CUDA tensors");
+  auto starts = [](const Tensor& t, int64_t n, at::ScalarType type) {
+    return t.is_cuda() && t.scalar_type() == type && t.is_contiguous() && t.numel() >= n && reinterpret_cast<uintptr_t>(t.data_ptr()) % 16 == 0;
+  };
+  TORCH_CHECK(tokens >= 0 && heads > 0 && D > 0 && stride_y == heads * D, "norm_rope: at least one head, y and dy dense");
+  TORCH_CHECK(x.is_cuda() && x.scalar_type() == at::kBFloat16 && x.numel() == tokens * heads * D && token_stride(x) >= 0 &&
+              stride_x == token_stride(x), "norm_rope: bf16 x of dense heads on 16-byte boundaries, and its token stride");
+  TORCH_CHECK(starts(y, tokens * heads * D, at::kBFloat16) && (!bwd || dy.has_value()) && (!dy.has_value() || starts(*dy, tokens * heads * D, at::kBFloat16)),
+              "norm_rope: y and dy are dense bf16 of x's size on 16-byte boundaries");
+  TORCH_CHECK(starts(cos, tokens * (D / 2), at::kFloat) && starts(sin, tokens * (D / 2), at::kFloat), "norm_rope: cos and sin are fp32 [tokens, D / 2] on 16-byte boundaries");
   c10::cuda::CUDAGuard guard(x.device());
   float* rs = rstd.has_value() ? rstd->data_ptr<float>() : nullptr;
   float* dwp = dw.has_value() ? dw->data_ptr<float>() : nullptr;
@@ -560,6 +584,7 @@ TORCH_LIBRARY(bux_b200, m) {
   m.def("quant_mxfp8(Tensor x, Tensor? row_index, Tensor? row_scale, Tensor? q_row, Tensor? sf_row, Tensor? q_col, Tensor? sf_col, int rows, int cols, int ld_col, int batch, int x_batch_stride) -> ()", &quant_mxfp8);
   m.def("quant_mxfp8_glu(Tensor h, Tensor? dout, Tensor? row_scale, Tensor? q_row, Tensor? sf_row, Tensor? q_col, Tensor? sf_col, int ld_col, int kind, float limit, float up_offset) -> ()", &quant_mxfp8_glu);
   m.def("quant_nvfp4(Tensor x, Tensor tensor_scale, Tensor(a!) packed, Tensor(b!) scales) -> ()", &quant_nvfp4);
+  m.def("token_stride(Tensor x) -> int", &token_stride);
   m.def("scale_to_bf16(Tensor src, Tensor scale, Tensor(a!) out) -> ()", &scale_to_bf16);
   m.def("ce_fwd_bwd(Tensor(a!) logits, Tensor targets, Tensor? mask, Tensor(b!) loss, Tensor? logz, float grad_scale, float z_weight, float softcap) -> ()", &ce_fwd_bwd);
   m.def("adamw(Tensor(a!) p, Tensor g, Tensor(b!) m, Tensor(c!) v, Tensor? m_sf, Tensor? v_sf, Tensor? shadow, Tensor? grad_scale, float lr, float b1, float b2, float eps, float wd, float bc1, float bc2, float grad_scale_const) -> ()", &adamw);

@@ -12,6 +12,9 @@ void gemm(const Tensor& a, const Tensor& b, Tensor& c, const std::optional<Tenso
           const std::optional<Tensor>& wait_flags, int64_t wait_epoch, int64_t wait_rows, int64_t m_rotate, bool wait_on_k, bool wait_on_n);
 void rmsnorm_fwd(const Tensor& x, const std::optional<Tensor>& w, Tensor& y, Tensor& rstd, double eps);
 void rmsnorm_bwd(const Tensor& x, const std::optional<Tensor>& w, const Tensor& dy, const Tensor& rstd, Tensor& dx, const std::optional<Tensor>& dw);
+// Elements between tokens of x [..., T, H, D] when heads are dense and the leading dimensions collapse
+// into one (a column slice of a fused projection), x starts on 16 bytes and every token too; else -1.
+int64_t token_stride(const Tensor& x);
 void norm_rope(bool bwd, const Tensor& x, const std::optional<Tensor>& w, const Tensor& cos, const Tensor& sin, Tensor& y,
                const std::optional<Tensor>& rstd, const std::optional<Tensor>& dy, const std::optional<Tensor>& dw, int64_t tokens,
                int64_t heads, int64_t D, int64_t stride_x, int64_t stride_y, double eps);

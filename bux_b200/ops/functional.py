@@ -82,7 +82,7 @@ class _NormRope(torch.autograd.Function):
     @staticmethod
     def forward(ctx, x, w, cos, sin, eps):
         K = _K()
-        xc = x if K.token_stride(x) is not None else x.contiguous()  # a slice of qkv is read in place
+        xc = K.walkable(x)  # a slice of qkv is read in place
         wf = None if w is None else w.float().contiguous()
         y, rstd = K.norm_rope_fwd(xc, wf, cos, sin, eps)
         ctx.save_for_backward(xc, w, cos, sin, rstd)
@@ -94,7 +94,7 @@ class _NormRope(torch.autograd.Function):
         K = _K()
         x, w, cos, sin, rstd = ctx.saved_tensors
         wf = None if w is None else w.float().contiguous()
-        dx, dw = K.norm_rope_bwd(x, wf, cos, sin, rstd, dy.contiguous(), ctx.eps)
+        dx, dw = K.norm_rope_bwd(K.walkable(x), wf, cos, sin, rstd, K.walkable(dy.contiguous()), ctx.eps)
         return dx, (None if w is None else dw.to(w.dtype)), None, None, None
 
 

@@ -266,14 +266,14 @@ def rmsnorm_bwd(x, w, dy, rstd, need_dw: bool = True):
 def token_stride(x) -> Optional[int]:
     """Elements between tokens of x [..., T, H, D] when heads are dense and the leading
     dimensions collapse into one (a column slice of a fused projection); else None."""
-    d, h = x.shape[-1], x.shape[-2]
-    if x.stride(-1) != 1 or x.stride(-2) != d or x.dim() < 3:
-        return None
-    step = x.stride(-3)
-    for i in range(x.dim() - 4, -1, -1):
-        if x.stride(i) != x.shape[i + 1] * x.stride(i + 1):
-            return None
-    return step if step % 8 == 0 and x.data_ptr() % 16 == 0 else None
+    step = ops().token_stride(x)
+    return None if step < 0 else step
+
+
+def walkable(x):
+    """x where the norm + RoPE kernel can read it in place, else a copy (`contiguous` would return x
+    itself whatever the strides of its dimensions of size 1 are, and wherever it starts)."""
+    return x if token_stride(x) is not None else x.clone(memory_format=torch.contiguous_format)
 
 
 def norm_rope_fwd(x, w, cos, sin, eps: float):

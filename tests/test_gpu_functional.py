@@ -324,3 +324,54 @@ def test_native_autograd_functions_refuse_and_recompute(cuda):
     with pytest.raises((NotImplementedError, RuntimeError)):
         with torch.autograd.forward_ad.dual_level():
             ops.rmsnorm(torch.autograd.forward_ad.make_dual(x.detach(), torch.ones_like(x)), w)
+
+
+@pytest.mark.parametrize("layout", ["tokens of one longer row", "one head, heads first", "between 16-byte boundaries", "gradient between them"])
+@pytest.mark.parametrize("weighted", [True, False])
+def test_norm_rope_of_layouts_that_only_look_dense(cuda, layout, weighted, monkeypatch):
+    """Tensors that PyTorch calls contiguous and the kernel cannot walk in place, through both forms of
+    the function, with gradients. Bounds: outputs are rounded to bf16 (2^-9), with one rotation more."""
+    from bux_b200.ops import functional as F
+
+    g = torch.Generator(device=cuda).manual_seed(4)
+    t, h, d = 60, 1 if layout.startswith("one head") else 4, 64
+    base = torch.randn(2 * 100 * 4 * d, generator=g, device=cuda).bfloat16()
+    if layout == "tokens of one longer row":
+        x = base[: 100 * h * d].view(1, 100, h, d)[:, :t]
+    elif h == 1:
+        x = base[: 2 * t * d].view(2, 1, t, d).transpose(1, 2)
+    else:
+        x = base[layout.startswith("between"):][: t * h * d].view(1, t, h, d)
+    w = torch.randn(d, generator=g, device=cuda)
+    cos, sin = ref.rope_tables(torch.arange(t, device=cuda)[None].expand(x.shape[0], t), d, 10000.0)
+    dy = torch.randn(x.numel() + 1, generator=g, device=cuda).bfloat16()[layout.startswith("gradient"):][: x.numel()].view(x.shape)
+    xr, wr = x.float().requires_grad_(), w.clone().requires_grad_()
+    want = ref.rmsnorm_rope(xr, wr, cos, sin, 1e-6) if weighted else ref.rope(xr, cos, sin)
+    want.backward(dy.float())
+    for python in (False, True):
+        with monkeypatch.context() as m:
+            if python:
+                m.setattr(F, "_native", lambda op: None)
+            xg, wg = x.detach().requires_grad_(), w.clone().requires_grad_()
+            y = ops.rmsnorm_rope(xg, wg if weighted else None, cos, sin, 1e-6)
+            grads = torch.autograd.grad(y, [xg, wg] if weighted else [xg], dy)
+        assert rel_err(y, want) < 4e-3 and rel_err(grads[0], xr.grad) < 4e-3
+        assert not weighted or rel_err(grads[1], wr.grad) < 1e-5
+
+
+def test_norm_rope_refuses_what_it_cannot_walk(cuda):
+    """The wrapper's own checks, below the functions that copy such tensors."""
+    from bux_b200.ops import kernels as K
+
+    x = torch.zeros(1, 8, 2, 64, device=cuda).bfloat16()
+    y, c = torch.empty_like(x), torch.zeros(8, 32, device=cuda)
+
+    def call(x=x, y=y, cos=c, sin=c, step=128, tokens=8, dy=None, bwd=False):
+        K.ops().norm_rope(bwd, x, None, cos, sin, y, None, dy, None, tokens, 2, 64, step, 128, 1e-6)
+
+    call()
+    bad = torch.zeros(8 * 2 * 64 + 1, device=cuda).bfloat16()[1:].view(1, 8, 2, 64)
+    for kw in ({"x": bad}, {"y": bad}, {"step": -1}, {"step": 64}, {"step": 256}, {"tokens": 9}, {"cos": c[:7]}, {"sin": c[:, :16]},
+               {"bwd": True}, {"bwd": True, "dy": bad}, {"x": x.float()}):
+        with pytest.raises(RuntimeError, match="norm_rope"):
+            call(**kw)
