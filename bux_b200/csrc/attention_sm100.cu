@@ -382,9 +382,11 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
       scale_o = keep;
     }
     const float inv = l > 0.f ? scale_o / l : 0.f;
-    // O as bf16 into the Q tile, in TMA's swizzled layout: every S has been computed. A warp's 32
-    // rows x 64 columns are one 4 KB slab; with heads of 64 the two halves fill one together.
-    const bool by_tma = q0 + x * QT + QT <= p.T;   // a tile that ends inside the row of tokens
+    // O as bf16 into the Q tile, in TMA's swizzled layout: the tile's last P·V is complete, so Q has been
+    // read. A warp's 32 rows x 64 columns are one 4 KB slab; with heads of 64 the two halves fill one
+    // together. A tile without keys has waited for nothing: its Q may still be on its way into that
+    // memory (the other tile's keys make the producer load both), so its zeros leave from registers.
+    const bool by_tma = done > 0 && q0 + x * QT + QT <= p.T;   // and the tile ends inside the row of tokens
     uint8_t* slab = sQ + x * Cfg::TILE_BYTES + (D == 128 ? half * 16384 : 0) + quad * 4096 + lane * 128;
     __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(p.o) + (((size_t)b * p.T + (q < p.T ? q : 0)) * p.H + h) * D + half * (D / 2);
     if (ok) {

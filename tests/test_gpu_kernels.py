@@ -480,6 +480,11 @@ def test_attention_fwd(cuda, d, h, g, t, window, sinks):
     (640, 640, True, 0, None, 40.0),     # scores of thousands: the rows' references move mid-way
     (256, 256, True, 0, 0.0, 1.0),       # every score equal
     (256, 256, True, 0, -0.1, 30.0),     # a negative scale
+    (256, 1, True, 0, None, 1.0),        # more queries than keys: the first tile of a pair sees none, the second one key
+    (383, 1, True, 0, None, 1.0),        # the last such length
+    (512, 256, True, 0, None, 1.0),      # a pair without keys, then one whose first tile has none
+    (640, 200, True, 64, None, 1.0),     # with a window, and a last pair of one tile
+    (1024, 700, False, 0, None, 1.0),    # no mask: every query sees every key
 ])
 @pytest.mark.parametrize("d", [64, 128])
 def test_attention_fwd_edges(cuda, d, t, s, causal, window, scale, spread):
