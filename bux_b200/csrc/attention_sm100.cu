@@ -305,7 +305,8 @@ attn_fwd_kernel(const __grid_constant__ AttnFwdParams p) {
 #pragma unroll
         for (int i = 0; i < 32; ++i) top[i & 3] = fmaxf(top[i & 3], fmaxf(score(checked, v[i], i), score(checked, w[i], 32 + i)));
         mx = fmaxf(fmaxf(top[0], top[1]), fmaxf(top[2], top[3]));
-        if (mx != -INFINITY) mx *= sc;
+        // no number (a scale that is none, 0 · inf) counts as no maximum: P then is no number by itself
+        if (mx != -INFINITY) mx = fmaxf(mx * sc, -INFINITY);
       };
       if (ok) {
         // two bodies: the checks would cost the tiles that need none two instructions per score

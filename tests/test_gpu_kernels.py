@@ -535,6 +535,24 @@ def test_attention_bwd(cuda, d, h, g, t, window, sinks):
         assert rel_err(dsk, sk.grad) < 3e-2
 
 
+@pytest.mark.parametrize("scale,peak", [(float("nan"), 1.0), (0.0, float("inf")), (0.0, float("nan")), (1.0, float("inf"))])
+@pytest.mark.parametrize("d", [64, 128])
+def test_attention_fwd_of_scores_that_are_no_numbers(cuda, d, scale, peak):
+    """A maximum that is no number is none, and no sign that a wait ran out: rows that see the NaN are
+    NaN, the rows before it are what they are without it, and the status word stays clear."""
+    from bux_b200.ops import kernels as K
+
+    torch.manual_seed(21)
+    q, k, v = (torch.rand(1, 300, 2, d, device=cuda).bfloat16() for _ in range(3))
+    clean, _ = K.attn_fwd(q, k, v, scale=0.0 if scale != scale else scale)
+    k[:, 200] = peak
+    got, _ = K.attn_fwd(q, k, v, scale=scale)
+    torch.cuda.synchronize()
+    K.check_status(cuda)
+    assert got[:, 200:].isnan().all()
+    assert got[:, :200].isnan().all() if scale != scale else torch.equal(got[:, :200], clean[:, :200])
+
+
 @pytest.mark.parametrize("d,h,g,t", [(64, 12, 4, 33), (128, 3, 1, 31), (64, 8, 8, 1), (128, 9, 3, 64)])
 def test_attention_sink_gradient_at_the_edges_of_its_tiles(cuda, d, h, g, t):
     """32 tokens x 8 heads go together in the kernel that forms delta and the sinks' gradient.
