@@ -1326,7 +1326,8 @@ __global__ void topk_rows_kernel(const float* __restrict__ scores, long* __restr
 // consecutive ranges and walk them 32 picks at a time, ranked by __match_any_sync, so picks of an
 // expert stay in order. It replaces a radix sort, a histogram with two host synchronisations and
 // some forty small launches: about 300 us with the waits for 131072 picks of 128 experts, now 20.
-// A pick outside [0, experts) is reported in the status word; its pos is -2 (see combine_rows).
+// A pick outside [0, experts) is reported in the status word (its count is then picks, not waits; the
+// host's text for this kernel's number says so); its pos is -2 (see combine_rows).
 constexpr int KID_PICKS = 12;
 constexpr int PICK_THREADS = 256;
 __global__ void __launch_bounds__(PICK_THREADS)

@@ -103,7 +103,9 @@ def sort_picks(experts: torch.Tensor, num_experts: int, align: int = 128):
 
     Returns (row_index int32[R] = source token of each padded row or -1,
     pos int32[T,k] = padded row of each pick, offsets int32[E+1]) where
-    R = T·k + E·(align-1) rounded up to `align` bounds the padded rows."""
+    R = T·k + E·(align-1) rounded up to `align` bounds the padded rows. A pick outside [0, E) raises
+    on the CPU; on the GPU, where the host does not wait for the picks, its pos is -2 and the device's
+    status word says so (`kernels.check_status`; the trainer reads it with its losses)."""
     return _sort_picks(experts, num_experts, align)[:3]
 
 
@@ -244,7 +246,9 @@ class _SortedExperts(torch.autograd.Function):
             # dh, and per row <da', glu(h)> = the gradient of that row's router weight
             dh, drs = K.glu_bwd(h, da, act, w_row, limit, up_offset)
             del da, h
-            dwts[c * tc:(c + 1) * tc] = drs[pos.reshape(-1).long()].view(pos.shape)
+            # a pick of no expert has no row (its pos is negative): its weight's gradient is NaN, like its output
+            at = pos.long()
+            dwts[c * tc:(c + 1) * tc] = drs[at.clamp_min(0)].masked_fill_(at < 0, float("nan"))
             if mx:
                 hq, hsf, htq, htsf = K.quant_mxfp8(dh, rowwise=True, colwise=True)
                 del dh
@@ -272,7 +276,8 @@ def moe_experts(x, w_gate_up, w_down, weights, experts, *, act: str = "swish",
                 limit: Optional[float] = None, up_offset: float = 0.0, fmt: str = "bf16", chunks: int = 1):
     """Routed experts on x [T,d]: out[t] = Σ_j weights[t,j] · expert_{experts[t,j]}(x[t]).
     w_gate_up [E, 2f, d] (gate rows first), w_down [E, d, f]. `chunks` walks the tokens in that
-    many equal ranges (``methods(moe_chunks=...)``)."""
+    many equal ranges (``methods(moe_chunks=...)``). A pick of no expert (see `sort_picks`) makes its
+    token's row of the output and of the gradient by x, and its weight's gradient, NaN."""
     e, f2, d = w_gate_up.shape
     f = f2 // 2
     mx = fmt in ("mxfp8", "mxfp8_2d")

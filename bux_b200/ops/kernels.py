@@ -47,22 +47,32 @@ def __getattr__(name: str):
 
 
 def status_word(device) -> torch.Tensor:
-    """Per-device int32[2] the kernels' bounded waits report into."""
+    """Per-device int32[2] the kernels report failures into (see `status_message`)."""
     key = torch.device(device).index or 0
     if key not in _status:
         _status[key] = torch.zeros(2, dtype=torch.int32, device=device)
     return _status[key]
 
 
+_PICKS = 12  # the kernel number under which `sort_picks` reports picks of no expert
+
+
+def status_message(code: int, count: int) -> str:
+    """What a status word that is not clear says."""
+    if code >> 24 == _PICKS:
+        return f"a router picked an expert that does not exist ({count} picks in total)"
+    return (f"a bounded device wait ran out (kernel {code >> 24}, site {(code >> 16) & 0xff}, "
+            f"block {code & 0xffff}; {count} waits in total)")
+
+
 def check_status(device, what: str = "kernel") -> None:
-    """Raise if any bounded wait of a kernel on `device` ran out (synchronises)."""
+    """Raise if a kernel on `device` reported a failure: a bounded wait that ran out, a router's pick
+    of no expert (synchronises)."""
     st = status_word(device)
     code, count = st.tolist()
     if code:
         st.zero_()
-        raise RuntimeError(
-            f"{what}: a bounded device wait ran out (kernel {code >> 24}, site {(code >> 16) & 0xff}, "
-            f"block {code & 0xffff}; {count} waits in total)")
+        raise RuntimeError(f"{what}: {status_message(code, count)}")
 
 
 # ------------------------------------------------------------------ GEMM

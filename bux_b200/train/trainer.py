@@ -46,7 +46,8 @@ def pick_device(spec: Optional[str] = None) -> torch.device:
 
 
 class KernelWaitError(RuntimeError):
-    """A kernel's bounded wait (on a peer's flag, a barrier) ran out during a step."""
+    """A kernel reported a failure during a step: a bounded wait (on a peer's flag, a barrier) ran
+    out, or a router picked an expert that does not exist."""
 
 
 class Timers:
@@ -349,11 +350,12 @@ class Trainer:
             self._prefixes = table.to(self.device)
         return self._prefixes
 
-    # ---- the kernels' bounded waits
+    # ---- what the kernels report
     def _snapshot_kernel_status(self) -> None:
         """Queue a copy of the device's status word (where a kernel's bounded wait records
-        that it ran out) into pinned host memory behind the step's work: reading it later
-        costs no synchronisation beyond the one the reader already made for that step."""
+        that it ran out, and the sort of a router's picks those of no expert) into pinned host
+        memory behind the step's work: reading it later costs no synchronisation beyond the one
+        the reader already made for that step."""
         if self.device.type != "cuda":
             return
         from ..ops import kernels as K
@@ -363,9 +365,10 @@ class Trainer:
         self._status_host.copy_(K.status_word(self.device), non_blocking=True)
 
     def check_kernels(self, what: str = "training step") -> None:
-        """Raise on every rank if a bounded device wait ran out on any rank in a step whose
-        results the host has already read (the log hook, before a checkpoint is written):
-        such a kernel returned without writing its output, so the state is not to be kept."""
+        """Raise on every rank if a bounded device wait ran out, or a router picked an expert that
+        does not exist, on any rank in a step whose results the host has already read (the log hook,
+        before a checkpoint is written): such a kernel returned without writing its output, or a
+        token's row is NaN, so the state is not to be kept."""
         if self._status_host is None:
             return
         code, count = (int(v) for v in self._status_host.tolist())
@@ -379,9 +382,8 @@ class Trainer:
         self.stopping = True
         K.status_word(self.device).zero_()
         self._status_host.zero_()
-        where = (f"kernel {code >> 24}, site {(code >> 16) & 0xff}, block {code & 0xffff}; {count} waits in total"
-                 if code else "on another rank")
-        raise KernelWaitError(f"{what}: a bounded device wait ran out ({where}); the step's results are stale")
+        said = K.status_message(code, count) if code else "a kernel on another rank reported a failure"
+        raise KernelWaitError(f"{what}: {said}; the step's results are stale")
 
     # ---- optimizer fused into the backward (gradients released as they are produced)
     def _install_release_hooks(self) -> None:

@@ -375,3 +375,34 @@ def test_norm_rope_refuses_what_it_cannot_walk(cuda):
                {"bwd": True}, {"bwd": True, "dy": bad}, {"x": x.float()}):
         with pytest.raises(RuntimeError, match="norm_rope"):
             call(**kw)
+
+
+@pytest.mark.parametrize("fmt", ["bf16", "mxfp8"])
+@pytest.mark.parametrize("bad", [-1, 4, 1 << 40])
+def test_a_pick_of_no_expert_spoils_its_own_token_alone(cuda, fmt, bad):
+    """Its row of the output and of dx, and its weight's gradient, are NaN; every other token is what
+    it is with valid picks; the status word says what happened."""
+    from bux_b200.ops import kernels as K
+
+    g = torch.Generator(device=cuda).manual_seed(6)
+    x, dy = (torch.randn(40, 128, generator=g, device=cuda).bfloat16() for _ in range(2))
+    w_gu = (torch.randn(4, 256, 128, generator=g, device=cuda) * 0.1).bfloat16()
+    w_down = (torch.randn(4, 128, 128, generator=g, device=cuda) * 0.1).bfloat16()
+    wts, good = torch.rand(40, 2, generator=g, device=cuda), torch.randint(0, 4, (40, 2), generator=g, device=cuda)
+
+    def run(picks):
+        xs = [t.detach().clone().requires_grad_() for t in (x, wts)]
+        y = ops.moe_experts(xs[0], w_gu, w_down, xs[1], picks, fmt=fmt)
+        return [y.detach(), *torch.autograd.grad(y, xs, dy)]
+
+    want = run(good)
+    picks = good.clone()
+    picks[7, 1] = bad
+    got = run(picks)
+    with pytest.raises(RuntimeError, match=r"does not exist \(1 picks"):
+        K.check_status(cuda)
+    rest = torch.arange(40, device=cuda) != 7
+    for a, b in zip(got, want):
+        assert torch.equal(a[rest], b[rest])
+    assert got[0][7].isnan().all() and got[1][7].isnan().all()
+    assert got[2][7, 1].isnan() and got[2][7, 0] == want[2][7, 0]

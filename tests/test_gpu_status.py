@@ -62,6 +62,20 @@ def test_trainer_reports_a_wait_that_ran_out(cuda):
     K.check_status(cuda, "test")
 
 
+def test_trainer_reports_a_pick_of_no_expert(cuda):
+    from bux_b200.lang import compile_runs
+    from bux_b200.ops import kernels as K
+    from bux_b200.train.trainer import KernelWaitError, Trainer
+
+    tr = Trainer(compile_runs(SRC, filename="s.bux")[0], device=cuda)
+    feed = iter(tr.batches())
+    K.sort_picks(torch.tensor([[0], [4]], device=cuda), 4, 1, 2)
+    tr.train_step(next(feed))["loss"].item()
+    with pytest.raises(KernelWaitError, match="an expert that does not exist"):
+        tr.check_kernels("step 1")
+    K.check_status(cuda, "test")
+
+
 def test_packed_rows_are_masked_by_document_on_the_gpu(cuda):
     """A row packed with several documents trains like those documents apart: position
     ids that restart mark the boundaries, and the trainer must turn them into segment
