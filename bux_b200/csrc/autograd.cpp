@@ -35,6 +35,7 @@ Tensor fp32_like(const Tensor& t, at::IntArrayRef shape) { return at::empty(shap
 // ------------------------------------------------------------------ RMSNorm
 struct RMSNorm : torch::autograd::Function<RMSNorm> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const OptTensor& w, double eps) {
+    TORCH_CHECK(x.dim() > 0 && x.size(-1) > 0, "rmsnorm: rows of at least one element");
     const Tensor xc = x.contiguous();
     Tensor y = at::empty(xc.sizes(), xc.options()), rstd = fp32_like(xc, {xc.numel() / xc.size(-1)});
     rmsnorm_fwd(xc, f32(w), y, rstd, eps);
@@ -63,6 +64,7 @@ Tensor walkable(const Tensor& x) {
 
 struct NormRope : torch::autograd::Function<NormRope> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const OptTensor& w, const Tensor& cos, const Tensor& sin, double eps) {
+    TORCH_CHECK(x.dim() >= 3 && x.size(-1) > 0 && x.size(-2) > 0, "norm_rope: x is [..., tokens, heads, D], of at least one head");
     const Tensor xc = walkable(x);
     const int64_t d = xc.size(-1), h = xc.size(-2), tokens = xc.numel() / (h * d);
     const Tensor c = cos.reshape({-1, d / 2}).to(at::kFloat).contiguous(), s = sin.reshape({-1, d / 2}).to(at::kFloat).contiguous();

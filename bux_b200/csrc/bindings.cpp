@@ -98,7 +98,7 @@ void gemm(const Tensor& a, const Tensor& b, Tensor& c, const c10::optional<Tenso
 void rmsnorm_fwd(const Tensor& x, const c10::optional<Tensor>& w, Tensor& y, Tensor& rstd, double eps) {
   check_cuda(x, "x"); check_cuda(y, "y");
   const int d = (int)x.size(-1);
-  TORCH_CHECK(d % 8 == 0 && x.scalar_type() == at::kBFloat16, "rmsnorm: bf16, width % 8 == 0");
+  TORCH_CHECK(d > 0 && d % 8 == 0 && x.scalar_type() == at::kBFloat16, "rmsnorm: bf16, width % 8 == 0 and not 0");
   c10::cuda::CUDAGuard guard(x.device());
   bux::rmsnorm_fwd(x.data_ptr(), opt_f32(w), y.data_ptr(), rstd.data_ptr<float>(), x.numel() / d, d, (float)eps, stream_of(x));
 }
@@ -106,6 +106,7 @@ void rmsnorm_bwd(const Tensor& x, const c10::optional<Tensor>& w, const Tensor& 
                  Tensor& dx, const c10::optional<Tensor>& dw) {
   check_cuda(x, "x"); check_cuda(dy, "dy"); check_cuda(dx, "dx");
   const int d = (int)x.size(-1);
+  TORCH_CHECK(d > 0, "rmsnorm: rows of at least one element");
   c10::cuda::CUDAGuard guard(x.device());
   float* dwp = dw.has_value() ? dw->data_ptr<float>() : nullptr;
   Tensor part;
@@ -160,7 +161,7 @@ void norm_rope(bool bwd, const Tensor& x, const c10::optional<Tensor>& w, const 
 void glu_fwd(const Tensor& h, Tensor& out, const c10::optional<Tensor>& row_scale, int64_t kind, double limit, double up_offset) {
   check_cuda(h, "h"); check_cuda(out, "out");
   const int f = (int)out.size(-1);
-  TORCH_CHECK(h.size(-1) == 2 * f && f % 8 == 0, "glu: h is [rows, 2f], f % 8 == 0");
+  TORCH_CHECK(f > 0 && h.size(-1) == 2 * f && f % 8 == 0, "glu: h is [rows, 2f], f % 8 == 0 and not 0");
   c10::cuda::CUDAGuard guard(h.device());
   bux::glu_fwd(h.data_ptr(), out.data_ptr(), opt_f32(row_scale), out.numel() / f, f, (int)kind, (float)limit, (float)up_offset, stream_of(h));
 }
@@ -168,6 +169,7 @@ void glu_bwd(const Tensor& h, const Tensor& dout, Tensor& dh, const c10::optiona
              const c10::optional<Tensor>& d_row_scale, int64_t kind, double limit, double up_offset) {
   check_cuda(h, "h"); check_cuda(dout, "dout"); check_cuda(dh, "dh");
   const int f = (int)dout.size(-1);
+  TORCH_CHECK(f > 0, "glu: rows of at least one element");
   c10::cuda::CUDAGuard guard(h.device());
   float* drs = d_row_scale.has_value() ? d_row_scale->data_ptr<float>() : nullptr;
   bux::glu_bwd(h.data_ptr(), dout.data_ptr(), dh.data_ptr(), opt_f32(row_scale), drs, dout.numel() / f, f, (int)kind, (float)limit, (float)up_offset, stream_of(h));

@@ -406,3 +406,15 @@ def test_a_pick_of_no_expert_spoils_its_own_token_alone(cuda, fmt, bad):
         assert torch.equal(a[rest], b[rest])
     assert got[0][7].isnan().all() and got[1][7].isnan().all()
     assert got[2][7, 1].isnan() and got[2][7, 0] == want[2][7, 0]
+
+
+def test_rows_without_elements_are_refused(cuda):
+    """An exception, where a division by the width or the head count would end the process."""
+    empty = torch.empty(4, 0, device=cuda, dtype=torch.bfloat16)
+    with pytest.raises(RuntimeError, match="rmsnorm"):
+        ops.rmsnorm(empty, None)
+    with pytest.raises(RuntimeError, match="glu"):
+        ops.glu(empty)
+    table = torch.zeros(1, 3, 32, device=cuda)
+    with pytest.raises(RuntimeError, match="norm_rope"):
+        ops.rope(torch.empty(1, 3, 0, 64, device=cuda, dtype=torch.bfloat16), table, table)
