@@ -418,3 +418,17 @@ def test_rows_without_elements_are_refused(cuda):
     table = torch.zeros(1, 3, 32, device=cuda)
     with pytest.raises(RuntimeError, match="norm_rope"):
         ops.rope(torch.empty(1, 3, 0, 64, device=cuda, dtype=torch.bfloat16), table, table)
+
+
+def test_cross_entropy_head_takes_a_batch_of_gradients(cuda):
+    """Several incoming gradients at once, as `jacobian(vectorize=True)` sends them: each one's result."""
+    g = torch.Generator(device=cuda).manual_seed(7)
+    x = torch.randn(9, 64, generator=g, device=cuda).bfloat16().requires_grad_()
+    w = torch.randn(128, 64, generator=g, device=cuda).bfloat16().requires_grad_()
+    tgt = torch.randint(0, 128, (9,), generator=g, device=cuda)
+    scales = torch.tensor([1.0, 0.37, -2.0], device=cuda)
+    many = torch.autograd.grad(ops.cross_entropy_head(x, w, tgt)[0], [x, w], scales, is_grads_batched=True)
+    for i, s in enumerate(scales):
+        one = torch.autograd.grad(ops.cross_entropy_head(x, w, tgt)[0], [x, w], s)
+        for a, b in zip(many, one):
+            assert a[i].dtype == b.dtype and torch.equal(a[i], b)
