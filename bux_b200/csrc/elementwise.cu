@@ -640,13 +640,13 @@ __device__ __forceinline__ int qtile_at(int row, int chunk) {
   const int g = (((row >> 5) & 3) << 1) | (row & 1);
   return row * QT + (((chunk & 8) | ((chunk ^ g ^ ((chunk >> 3) << 1)) & 7)) << 3);
 }
-// The largest magnitude of 32 bf16 values in 16 words, two at a time (a NaN never wins).
+// The largest magnitude of 32 bf16 values in 16 words, two at a time (a NaN never wins: 0 where all are).
 __device__ __forceinline__ float amax32(const uint32_t (&w)[16]) {
   uint32_t m = w[0] & 0x7fff7fffu;
 #pragma unroll
   for (int j = 1; j < 16; ++j) asm("max.bf16x2 %0, %1, %2;" : "=r"(m) : "r"(m), "r"(w[j] & 0x7fff7fffu));
   const float2 t = unpack_bf16(m);
-  return fmaxf(t.x, t.y);
+  return fmaxf(fmaxf(t.x, t.y), 0.f);
 }
 // 1 / 2^(e - 127) as bf16 (exact; e = 254 gives bf16's 2^-127).
 __device__ __forceinline__ unsigned short e8m0_inv_bf16(uint8_t e) {

@@ -149,6 +149,24 @@ def test_grouped_gemm_contraction(cuda):
     assert first[1].abs().max() == 0   # the empty group stays zero
 
 
+def test_quant_mxfp8_of_blocks_without_numbers(cuda):
+    """A block of nothing but NaN has the scale of an empty one (byte 0, 2^-127), one with a single
+    number that number's, one with an infinity the largest; every NaN stays one."""
+    from bux_b200.ops import kernels as K
+
+    x = torch.full((128, 128), float("nan"), device=cuda).bfloat16()
+    x[0, 32], x[1, 64], x[2, 96] = 448.0, -3.5, float("inf")
+    want = torch.zeros(128, 4, dtype=torch.uint8, device=cuda)
+    want[0, 1], want[1, 2], want[2, 3] = 127, 120, 254
+    q, sf, qt, sft = K.quant_mxfp8(x, rowwise=True, colwise=True)
+    assert torch.equal(ref.unswizzle_scales(sf, 128, 4), want)
+    assert torch.equal(q.float().isnan(), x.isnan()) and torch.equal(qt.float().isnan(), x.t().isnan())
+    assert q[0, 32].float() == 448 and q[1, 64].float() == -448 and q[2, 96].float() == 448
+    cols = torch.zeros(128, 4, dtype=torch.uint8, device=cuda)
+    cols[32, 0], cols[64, 0], cols[96, 0] = 127, 120, 254
+    assert torch.equal(ref.unswizzle_scales(sft, 128, 4), cols)
+
+
 @pytest.mark.parametrize("m,n", [(32, 8), (160, 264), (224, 648), (72, 96)])
 @pytest.mark.parametrize("dtype,accumulate", [(torch.bfloat16, False), (torch.float32, False), (torch.float32, True)])
 def test_grouped_contraction_with_ragged_outputs(cuda, m, n, dtype, accumulate):
