@@ -94,6 +94,11 @@ void gemm(const Tensor& a, const Tensor& b, Tensor& c, const c10::optional<Tenso
   TORCH_CHECK(err == nullptr, "bux gemm: ", err);
 }
 
+std::vector<int64_t> gemm_plan(int64_t kind, int64_t M, int64_t N, int64_t K) {
+  const bux::GemmPlan plan = bux::gemm_plan((int)kind, M, N, K, 0, true);
+  return {plan.bn, plan.splits};
+}
+
 // ------------------------------------------------------------------ norms
 void rmsnorm_fwd(const Tensor& x, const c10::optional<Tensor>& w, Tensor& y, Tensor& rstd, double eps) {
   check_cuda(x, "x"); check_cuda(y, "y");
@@ -586,6 +591,7 @@ TORCH_LIBRARY(bux_b200, m) {
   m.def("quant_mxfp8(Tensor x, Tensor? row_index, Tensor? row_scale, Tensor? q_row, Tensor? sf_row, Tensor? q_col, Tensor? sf_col, int rows, int cols, int ld_col, int batch, int x_batch_stride) -> ()", &quant_mxfp8);
   m.def("quant_mxfp8_glu(Tensor h, Tensor? dout, Tensor? row_scale, Tensor? q_row, Tensor? sf_row, Tensor? q_col, Tensor? sf_col, int ld_col, int kind, float limit, float up_offset) -> ()", &quant_mxfp8_glu);
   m.def("quant_nvfp4(Tensor x, Tensor tensor_scale, Tensor(a!) packed, Tensor(b!) scales) -> ()", &quant_nvfp4);
+  m.def("gemm_plan(int kind, int M, int N, int K) -> int[]", &gemm_plan);
   m.def("token_stride(Tensor x) -> int", &token_stride);
   m.def("scale_to_bf16(Tensor src, Tensor scale, Tensor(a!) out) -> ()", &scale_to_bf16);
   m.def("ce_fwd_bwd(Tensor(a!) logits, Tensor targets, Tensor? mask, Tensor(b!) loss, Tensor? logz, float grad_scale, float z_weight, float softcap) -> ()", &ce_fwd_bwd);

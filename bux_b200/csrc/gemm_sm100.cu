@@ -723,11 +723,12 @@ __global__ void __launch_bounds__(256) sum_splits_kernel(const float* __restrict
 }
 
 // One wave of 256-wide tiles costs 1, of 128-wide ones 0.62 (more operand traffic per product: 8192^3
-// 0.54, 32768 x 5120 x 2048 0.62, 16384 x 14336 x 4096 0.65 of the wide tile's time), so the narrow tile is taken where it
-// saves enough of a last wave. Where even its tiles leave half of the SMs idle, the contraction is cut
-// as well, in ranges of at least four steps: a small product is a stream of its operands, and what
-// bounds it is how many SMs read. 16 x 6144 x 4096 (48 narrow tiles): 23.4 us with 24 wide tiles (29 with cold operands), 14.5 in 3
-// ranges and their sum.
+// 0.54, 32768 x 5120 x 2048 0.62, 16384 x 14336 x 4096 0.65 of the wide tile's time), so the narrow tile is
+// taken where it saves enough of a last wave. Where even its tiles leave half of the SMs idle, the
+// contraction is cut as well, in ranges of at least four steps (the last may be shorter, none is
+// empty): a small product is a stream of its operands, and what bounds it is how many SMs read.
+// 16 x 6144 x 4096 (48 narrow tiles): 23.4 us with 24 wide tiles (29 with cold operands), 14.5 in 3 ranges
+// and their sum.
 GemmPlan gemm_plan(int kind, long M, long N, long K, int sms, bool may_split) {
   if (sms <= 0) sms = 148;
   const long mt = (M + BM - 1) / BM, wide = mt * ((N + 255) / 256), narrow = mt * ((N + 127) / 128);
@@ -735,8 +736,10 @@ GemmPlan gemm_plan(int kind, long M, long N, long K, int sms, bool may_split) {
   GemmPlan plan{256, 1};
   if (!wide_fits || (narrow + sms - 1) / sms * 0.62 < (double)((wide + sms - 1) / sms)) plan.bn = 128;
   const long steps = (K + (kind == KIND_BF16 ? 63 : 127)) / (kind == KIND_BF16 ? 64 : 128);
-  if (may_split && plan.bn == 128 && narrow > 0 && narrow * 2 <= sms && steps >= 8)
-    plan.splits = (int)(sms / narrow < steps / 4 ? sms / narrow : steps / 4);
+  if (may_split && plan.bn == 128 && narrow > 0 && narrow * 2 <= sms && steps >= 8) {
+    const long most = sms / narrow < steps / 4 ? sms / narrow : steps / 4, per = (steps + most - 1) / most;
+    plan.splits = (int)((steps + per - 1) / per);
+  }
   return plan;
 }
 

@@ -242,7 +242,7 @@ def test_norm_rope_odd_heads(cuda, tokens, heads, d):
     assert rel_err(y, want) < 4e-3 and rel_err(dx, xr.grad) < 4e-3 and rel_err(dw, wr.grad) < 1e-5
 
 
-@pytest.mark.parametrize("m,n,k", [(1, 8, 512), (16, 6144, 4096), (130, 136, 1000), (128, 256, 2048), (3, 2048, 568), (509, 1024, 3072)])
+@pytest.mark.parametrize("m,n,k", [(1, 8, 512), (16, 6144, 4096), (130, 136, 1000), (128, 256, 2048), (3, 2048, 568), (509, 1024, 3072), (16, 256, 2880)])
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_small_products_are_split(cuda, m, n, k, a_mn, b_mn, dtype):
