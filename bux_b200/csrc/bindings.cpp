@@ -96,7 +96,7 @@ void gemm(const Tensor& a, const Tensor& b, Tensor& c, const c10::optional<Tenso
 
 std::vector<int64_t> gemm_plan(int64_t kind, int64_t M, int64_t N, int64_t K) {
   const bux::GemmPlan plan = bux::gemm_plan((int)kind, M, N, K, 0, true);
-  return {plan.bn, plan.splits};
+  return {plan.bn, plan.splits, kind == bux::KIND_BF16 && plan.bn == 256 && plan.splits == 1 && bux::gemm_pairs(M, N, K)};
 }
 
 // ------------------------------------------------------------------ norms

@@ -730,7 +730,7 @@ __global__ void __launch_bounds__(256) sum_splits_kernel(const float* __restrict
 // 16 x 6144 x 4096 (48 narrow tiles): 23.4 us with 24 wide tiles (29 with cold operands), 14.5 in 3 ranges
 // and their sum.
 GemmPlan gemm_plan(int kind, long M, long N, long K, int sms, bool may_split) {
-  if (sms <= 0) sms = 148;
+  if (sms <= 0) sms = GEMM_SMS;
   const long mt = (M + BM - 1) / BM, wide = mt * ((N + 255) / 256), narrow = mt * ((N + 127) / 128);
   const bool wide_fits = kind == KIND_BF16 || N % 256 == 0;
   GemmPlan plan{256, 1};
@@ -765,16 +765,21 @@ static const char* launch_kernel(const GemmArgs& a, const GemmParams& p, int sms
 }
 
 
-// Pairs take the dense bf16 products of wide tiles that fill them: at least a wave of 256 x 256 tiles
-// (with fewer neither is better: 64 tiles of 2048 x 2048 x 4096 30 us both, 20 of 512 x 4096 x 4096 25 and 27),
-// C where TMA can store it, nothing arriving from other GPUs.
-constexpr int PAIR_MIN_TILES = 74;
+// Pairs take the products of wide tiles that fill them: at least a wave of 256 x 256 tiles (with fewer
+// neither is better: 64 tiles of 2048 x 2048 x 4096 30 us both, 20 of 512 x 4096 x 4096 25 and 27); no more
+// waves than 128 x 256 tiles on single CTAs take, which is what rows that fill only half of the pairs' tiles and last
+// waves cost (128 x 18952 x 2048: 2 waves for 1, 35.7 us for 29.6; 776 x 5120 x 2048 30.7 for 24.6,
+// 384 x 151936 x 2048 214 for 193); and contractions of at least eight steps, since a pair's tile starts and ends
+// with both CTAs waiting for one another (14336 x 4096 x 128 43 us for 35, x 384 51 for 49, x 512 the same).
+bool gemm_pairs(long M, long N, long K) {
+  constexpr long PAIRS = GEMM_SMS / 2;
+  const long tiles = (M + 255) / 256 * ((N + 255) / 256), single = (M + BM - 1) / BM * ((N + 255) / 256);
+  return K >= 8 * PairCfg::BK && tiles >= PAIRS && (tiles + PAIRS - 1) / PAIRS <= (single + GEMM_SMS - 1) / GEMM_SMS;
+}
+// And nothing arrives from other GPUs, no SMs are kept free. (C has to be where TMA can store it.)
 static bool takes_pairs(const GemmArgs& a) {
-  const long tiles = (long)((a.M + 255) / 256) * ((a.N + 255) / 256);
-  const int c_elem = (a.out_kind == OUT_BF16 || a.out_kind == OUT_BF16_ACC) ? 2 : 4;
   return a.kind == KIND_BF16 && a.mode == MODE_DENSE && a.bn == 256 && a.splits <= 1 && a.wait_flags == nullptr &&
-         a.m_rotate == 0 && a.sms <= 0 && a.K > 0 && tiles >= PAIR_MIN_TILES && a.ldc * c_elem % 16 == 0 &&
-         reinterpret_cast<uintptr_t>(a.c) % 16 == 0;
+         a.m_rotate == 0 && a.sms <= 0 && gemm_pairs(a.M, a.N, a.K);
 }
 
 template <bool A_MN, bool B_MN>
@@ -786,8 +791,7 @@ static const char* launch_pair_as(const GemmParams& p, int ctas, cudaStream_t st
   return cudaGetLastError() == cudaSuccess ? nullptr : "gemm kernel launch failed";
 }
 static const char* launch_pair(const GemmArgs& a, const GemmParams& p, cudaStream_t stream) {
-  const long tiles = (long)((a.M + 255) / 256) * ((a.N + 255) / 256);
-  const int ctas = tiles < 74 ? 2 * (int)tiles : 148;
+  constexpr int ctas = GEMM_SMS;   // `gemm_pairs`: every pair has a tile
   if (a.a_mn) return a.b_mn ? launch_pair_as<true, true>(p, ctas, stream) : launch_pair_as<true, false>(p, ctas, stream);
   return a.b_mn ? launch_pair_as<false, true>(p, ctas, stream) : launch_pair_as<false, false>(p, ctas, stream);
 }
@@ -795,7 +799,7 @@ static const char* launch_pair(const GemmArgs& a, const GemmParams& p, cudaStrea
 static const char* sum_splits(const GemmArgs& a, cudaStream_t stream) {
   const bool vec = a.N % 4 == 0;
   const long threads = (long)a.M * a.N / (vec ? 4 : 1);
-  const int grid = (int)((threads + 255) / 256 < 148 * 8 ? (threads + 255) / 256 : 148 * 8);
+  const int grid = (int)((threads + 255) / 256 < GEMM_SMS * 8 ? (threads + 255) / 256 : GEMM_SMS * 8);
   if (a.out_kind == OUT_BF16) {
     if (vec) sum_splits_kernel<__nv_bfloat16, 4><<<grid, 256, 0, stream>>>(a.partial, (__nv_bfloat16*)a.c, a.M, a.N, a.ldc, a.splits);
     else sum_splits_kernel<__nv_bfloat16, 1><<<grid, 256, 0, stream>>>(a.partial, (__nv_bfloat16*)a.c, a.M, a.N, a.ldc, a.splits);
@@ -827,17 +831,8 @@ const char* gemm_launch(const GemmArgs& args, cudaStream_t stream) {
   const int elem = a.kind == KIND_BF16 ? 2 : 1;
   const int bk = a.kind == KIND_BF16 ? 64 : 128;
   const int bn = a.bn;
-  const bool pair = takes_pairs(a);
   if (a.kind == KIND_MXFP8 && (a.a_mn || a.b_mn)) return "mxfp8 operands are K-major";
   if (a.kind == KIND_MXFP8 && (p.k_total % 128 != 0)) return "mxfp8 K must be a multiple of 128";
-  const char* err;
-  // A: K-major [a_rows, K] box {bk, 128};  MN-major stored [K, a_rows] box {64, bk}
-  if (a.a_mn) err = make_tmap_2d(&p.tmap_a, a.a, elem, a.a_outer, a.a_inner, a.lda_bytes, 64, bk);
-  else        err = make_tmap_2d(&p.tmap_a, a.a, elem, a.a_outer, a.a_inner, a.lda_bytes, bk, BM);
-  if (err) return err;
-  if (a.b_mn) err = make_tmap_2d(&p.tmap_b, a.b, elem, a.b_outer, a.b_inner, a.ldb_bytes, 64, bk);
-  else        err = make_tmap_2d(&p.tmap_b, a.b, elem, a.b_outer, a.b_inner, a.ldb_bytes, bk, pair ? 128 : bn);
-  if (err) return err;
   p.tma_store = 0;
   const int c_elem = (a.out_kind == OUT_BF16 || a.out_kind == OUT_BF16_ACC) ? 2 : 4;
   if (a.ldc * c_elem % 16 == 0 && reinterpret_cast<uintptr_t>(a.c) % 16 == 0 &&
@@ -851,11 +846,17 @@ const char* gemm_launch(const GemmArgs& args, cudaStream_t stream) {
     if (make_tmap_2d(&p.tmap_c, a.c, c_elem, rows, (uint64_t)a.N, (uint64_t)a.ldc * c_elem, 128 / c_elem, 32) == nullptr)
       p.tma_store = 1;
   }
-  if (pair) {
-    if (!p.tma_store) return "a product on CTA pairs stores by TMA";
-    return launch_pair(a, p, stream);
-  }
-  int sms = a.sms > 0 ? a.sms : 148;
+  const bool pair = p.tma_store && takes_pairs(a);
+  const char* err;
+  // A: K-major [a_rows, K] box {bk, 128};  MN-major stored [K, a_rows] box {64, bk}
+  if (a.a_mn) err = make_tmap_2d(&p.tmap_a, a.a, elem, a.a_outer, a.a_inner, a.lda_bytes, 64, bk);
+  else        err = make_tmap_2d(&p.tmap_a, a.a, elem, a.a_outer, a.a_inner, a.lda_bytes, bk, BM);
+  if (err) return err;
+  if (a.b_mn) err = make_tmap_2d(&p.tmap_b, a.b, elem, a.b_outer, a.b_inner, a.ldb_bytes, 64, bk);
+  else        err = make_tmap_2d(&p.tmap_b, a.b, elem, a.b_outer, a.b_inner, a.ldb_bytes, bk, pair ? 128 : bn);
+  if (err) return err;
+  if (pair) return launch_pair(a, p, stream);
+  int sms = a.sms > 0 ? a.sms : GEMM_SMS;
   if (a.mode == MODE_DENSE) {   // no block without a tile
     const long tiles = (long)((a.M + BM - 1) / BM) * ((a.N + bn - 1) / bn) * p.splits;
     if (tiles < sms) sms = tiles > 0 ? (int)tiles : 1;

@@ -58,6 +58,10 @@ struct GemmArgs {
   bool wait_on_n = false;  // the senders write row blocks of B (sharded weights arriving from their owners)
 };
 
+constexpr int GEMM_SMS = 148;   // SMs of the chip: a launch's blocks, and twice its CTA pairs
+
+// Whether a dense bf16 product of 256-wide tiles runs on CTA pairs.
+bool gemm_pairs(long M, long N, long K);
 // Tile width and number of contraction ranges for a dense product, from how full the SMs get.
 struct GemmPlan { int bn, splits; };
 GemmPlan gemm_plan(int kind, long M, long N, long K, int sms, bool may_split);

@@ -14,10 +14,21 @@ def test_no_range_of_the_contraction_is_empty(kind, step):
     shapes += [(rng.randint(1, 600), 128 * rng.randint(1, 40), 8 * rng.randint(1, 4000)) for _ in range(500)]
     split = 0
     for m, n, k in shapes:
-        _, splits = K.ops().gemm_plan(kind, m, n, k)
+        _, splits, _ = K.ops().gemm_plan(kind, m, n, k)
         steps = -(-k // step)
         per = -(-steps // splits)
         assert (splits - 1) * per < steps, (m, n, k, splits)
         assert splits == 1 or (per >= 4 and splits * -(-m // 128) * -(-n // 128) <= 148)
         split += splits > 1
     assert split > 20
+
+
+@pytest.mark.parametrize("m,n,k,pairs", [
+    (8192, 14336, 4096, True), (4096, 151936, 2048, True), (256, 151936, 2048, True),
+    (128, 18952, 2048, False), (16, 201088, 2880, False), (384, 151936, 2048, False),   # rows fill half of the tiles
+    (776, 5120, 2048, False), (640, 14336, 4096, False),                                # a wave more
+    (14336, 4096, 448, False), (14336, 4096, 512, True),                                # short contractions
+    (2048, 2048, 4096, False)])                                                         # under a wave
+def test_pairs_of_sms_take_what_fills_them(m, n, k, pairs):
+    assert K.ops().gemm_plan(K.KIND_BF16, m, n, k)[2] == pairs
+    assert not K.ops().gemm_plan(K.KIND_MXFP8, m, n, k)[2]

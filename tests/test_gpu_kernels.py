@@ -262,12 +262,14 @@ def test_small_products_are_split(cuda, m, n, k, a_mn, b_mn, dtype):
     assert torch.equal(out, again)
 
 
-@pytest.mark.parametrize("m,n,k", [(2568, 2056, 200), (4224, 1288, 64), (8, 18952, 72), (2048, 2560, 1024)])
+@pytest.mark.parametrize("m,n,k", [(2568, 2056, 584), (4224, 1288, 512), (136, 18952, 520), (2048, 2560, 1024),
+                                   (2568, 2056, 200), (4224, 1288, 64), (8, 18952, 72)])
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, False), (True, True)])
 @pytest.mark.parametrize("out", ["bf16", "f32", "f32 +="])
 def test_products_on_pairs_of_sms(cuda, m, n, k, a_mn, b_mn, out):
-    """Enough 256 x 256 tiles for CTA pairs: tiles of which one CTA's rows or columns lie outside, one
-    step and ragged steps of the contraction, all layouts, stores and additions. Bounds as above."""
+    """Enough 256 x 256 tiles for CTA pairs: tiles of which one CTA's rows or columns lie outside, the
+    shortest contraction and ragged steps, all layouts, stores and additions. The last three are what
+    pairs leave to single CTAs: short contractions, rows that fill a sliver. Bounds as above."""
     from bux_b200.ops import kernels as K
 
     torch.manual_seed(18)
