@@ -32,3 +32,11 @@ def test_no_range_of_the_contraction_is_empty(kind, step):
 def test_pairs_of_sms_take_what_fills_them(m, n, k, pairs):
     assert K.ops().gemm_plan(K.KIND_BF16, m, n, k)[2] == pairs
     assert not K.ops().gemm_plan(K.KIND_MXFP8, m, n, k)[2]
+
+
+@pytest.mark.parametrize("kind,m,n,k,splits", [
+    (K.KIND_BF16, 16, 6144, 4096, 3), (K.KIND_BF16, 1, 2048, 2880, 9), (K.KIND_MXFP8, 16, 4096, 6144, 4),
+    (K.KIND_BF16, 128, 2048, 512, 1), (K.KIND_BF16, 16, 8192, 1024, 1), (K.KIND_MXFP8, 300, 1152, 2048, 1)])
+def test_short_contractions_are_not_split(kind, m, n, k, splits):
+    """The ranges have to save more than the second launch and the partial sums cost."""
+    assert K.ops().gemm_plan(kind, m, n, k)[1] == splits

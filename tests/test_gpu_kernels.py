@@ -242,12 +242,13 @@ def test_norm_rope_odd_heads(cuda, tokens, heads, d):
     assert rel_err(y, want) < 4e-3 and rel_err(dx, xr.grad) < 4e-3 and rel_err(dw, wr.grad) < 1e-5
 
 
-@pytest.mark.parametrize("m,n,k", [(1, 8, 512), (16, 6144, 4096), (130, 136, 1000), (128, 256, 2048), (3, 2048, 568), (509, 1024, 3072), (16, 256, 2880)])
+@pytest.mark.parametrize("m,n,k", [(1, 8, 512), (16, 6144, 4096), (130, 136, 1000), (128, 256, 2048), (3, 2048, 568), (509, 1024, 3072), (16, 256, 2880),
+                                   (1, 8, 2048), (130, 136, 2504), (3, 2048, 4088)])
 @pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_small_products_are_split(cuda, m, n, k, a_mn, b_mn, dtype):
-    """Products too small to fill the SMs: one row, ragged edges of the tiles and of the last range of
-    the contraction. Bounds: bf16 outputs are rounded once (2^-9); in fp32 the tensor core cuts its
+    """Products too small to fill the SMs, split and too short to be: one row, ragged edges of the tiles
+    and of the last range of the contraction. Bounds: bf16 outputs are rounded once (2^-9); in fp32 the tensor core cuts its
     accumulator's low bits once per 16 terms, 2^-23 of it each time (measured 1.4e-6 at k = 4096)."""
     from bux_b200.ops import kernels as K
 
@@ -281,7 +282,7 @@ def test_products_on_pairs_of_sms(cuda, m, n, k, a_mn, b_mn, out):
     assert rel_err(got, want + 1 if into is not None else want) < (4e-3 if out == "bf16" else 3e-6)
 
 
-@pytest.mark.parametrize("m,n,k", [(1, 128, 1024), (100, 384, 2048), (128, 256, 4096)])
+@pytest.mark.parametrize("m,n,k", [(1, 128, 1024), (100, 384, 2048), (128, 256, 4096), (1, 128, 4096), (100, 384, 6144)])
 def test_small_mxfp8_products_are_split(cuda, m, n, k):
     from bux_b200.ops import kernels as K
 
