@@ -593,30 +593,46 @@ glu_bwd_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restr
   }
 }
 
-// The same with the gradient of the row scale: a warp per row, so that the row's sum is one shuffle
+// The same with the gradient of the row scale: TPR threads per row, so that the row's sum is a
 // reduction and one store. (An atomic per eight columns queued f / 8 of them on one address:
-// 7200 rows of 2880 took 129 us, now 51; 147000 rows of 768 286, now 182.)
+// 7200 rows of 2880 took 129 us, a warp per row 51; 147456 rows of 768 312 and 182.)
+template <int TPR>
 __global__ void __launch_bounds__(256)
 glu_bwd_rows_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __restrict__ dout,
                     __nv_bfloat16* __restrict__ dh, const float* __restrict__ row_scale,
                     float* __restrict__ d_row_scale, long rows, int f, int kind, float limit, float up_offset) {
-  const int lane = threadIdx.x & 31, nvec = f / 8;
-  for (long row = (long)blockIdx.x * 8 + (threadIdx.x >> 5); row < rows; row += (long)gridDim.x * 8) {
-    const uint4* gp = reinterpret_cast<const uint4*>(h + row * 2 * f);
-    const uint4* dp = reinterpret_cast<const uint4*>(dout + row * f);
-    uint4* op = reinterpret_cast<uint4*>(dh + row * 2 * f);
-    const float rs = row_scale ? row_scale[row] : 1.f;
+  constexpr int RPB = 256 / TPR;   // rows a block works on at once
+  __shared__ float part[8];
+  const int li = threadIdx.x % TPR, nvec = f / 8;
+  // whole blocks iterate together: the reductions need every thread
+  for (long first = (long)blockIdx.x * RPB; first < rows; first += (long)gridDim.x * RPB) {
+    const long row = first + threadIdx.x / TPR;
     float ds = 0.f;
+    if (row < rows) {
+      const uint4* gp = reinterpret_cast<const uint4*>(h + row * 2 * f);
+      const uint4* dp = reinterpret_cast<const uint4*>(dout + row * f);
+      uint4* op = reinterpret_cast<uint4*>(dh + row * 2 * f);
+      const float rs = row_scale ? row_scale[row] : 1.f;
 #pragma unroll 3
-    for (int c = lane; c < nvec; c += 32) {
-      const uint4 gv = gp[c], uv = gp[nvec + c], dv = dp[c];
-      uint4 og, ou;
-      ds += glu_bwd_piece(gv, uv, dv, rs, kind, limit, up_offset, og, ou);
-      op[c] = og;
-      op[nvec + c] = ou;
+      for (int c = li; c < nvec; c += TPR) {
+        const uint4 gv = gp[c], uv = gp[nvec + c], dv = dp[c];
+        uint4 og, ou;
+        ds += glu_bwd_piece(gv, uv, dv, rs, kind, limit, up_offset, og, ou);
+        op[c] = og;
+        op[nvec + c] = ou;
+      }
     }
-    ds = warp_sum(ds);
-    if (lane == 0) d_row_scale[row] = ds;
+#pragma unroll
+    for (int o = (TPR < 32 ? TPR : 32) / 2; o > 0; o >>= 1) ds += __shfl_xor_sync(0xffffffffu, ds, o);
+    if (TPR > 32) {
+      if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ds;
+      __syncthreads();
+      ds = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) ds += part[w];
+      __syncthreads();
+    }
+    if (li == 0 && row < rows) d_row_scale[row] = ds;
   }
 }
 
@@ -1588,8 +1604,18 @@ void glu_fwd(const void* h, void* out, const float* row_scale, long rows, int f,
   glu_fwd_kernel<<<grid_for(rows * (f / 8), 256), 256, 0, s>>>((const __nv_bfloat16*)h, (__nv_bfloat16*)out, row_scale, rows, f, kind, limit, up_offset);
 }
 void glu_bwd(const void* h, const void* dout, void* dh, const float* row_scale, float* d_row_scale, long rows, int f, int kind, float limit, float up_offset, cudaStream_t s) {
-  if (d_row_scale)
-    glu_bwd_rows_kernel<<<grid_for(rows, 8, 148 * 16), 256, 0, s>>>((const __nv_bfloat16*)h, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dh, row_scale, d_row_scale, rows, f, kind, limit, up_offset);
+  if (d_row_scale) {
+#define GR_CASE(TPR_) glu_bwd_rows_kernel<TPR_><<<grid_for(rows, 256 / TPR_, 148 * 16), 256, 0, s>>>((const __nv_bfloat16*)h, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dh, row_scale, d_row_scale, rows, f, kind, limit, up_offset)
+    // A warp per row, but for rows that leave most of its lanes idle (65536 x 64: atomics 14.3 us, a warp
+    // 34.0, eight threads 16.4; 147456 x 8: 9.6, 64.6, 22.5 with eight) and for rows too few for their warps to fill
+    // the GPU (1 x 14336: 8.7, 52.9, a block per row 12.3; 1000 x 2880 73.9, 22.3, 14.3; from 4096 rows on
+    // a warp is no slower, and so at 2368 x 768).
+    if (rows <= 148 * 8) { if (f >= 768) GR_CASE(256); else GR_CASE(32); }
+    else if (f < 64) GR_CASE(1);
+    else if (f <= 128) GR_CASE(8);
+    else GR_CASE(32);
+#undef GR_CASE
+  }
   else
     glu_bwd_kernel<<<grid_for(rows * (f / 8), 256), 256, 0, s>>>((const __nv_bfloat16*)h, (const __nv_bfloat16*)dout, (__nv_bfloat16*)dh, row_scale, rows, f, kind, limit, up_offset);
 }

@@ -458,9 +458,11 @@ def test_a_pick_of_no_expert_is_reported(cuda):
         K.check_status(cuda)
 
 
-@pytest.mark.parametrize("rows,f", [(1, 8), (9, 248), (5, 264), (700, 768)])
+@pytest.mark.parametrize("rows,f", [(1, 8), (9, 248), (5, 264), (700, 768), (1300, 56), (1185, 64), (33, 128), (3, 136),
+                                    (40000, 128), (1184, 768), (1185, 776), (2, 14336)])
 def test_glu_backward_rows(cuda, rows, f):
-    """One warp per row: rows narrower than a warp's step and remainders of it. Bounds: gradients
+    """One, eight, 32 or 256 threads per row: rows narrower than their step, remainders of it, blocks
+    that walk several rows, and the widths and row counts where the split changes. Bounds: gradients
     are rounded to bf16 (2^-9); the row scale's is an fp32 sum."""
     from bux_b200.ops import kernels as K
 
