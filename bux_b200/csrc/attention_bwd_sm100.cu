@@ -29,52 +29,63 @@ constexpr int BWD_THREADS = 320;  // 8 softmax warps (two per TMEM lane quadrant
 constexpr float LOG2E_B = 1.4426950408889634f;
 
 // delta[b, h, t] = sum_d O·dO, and the sinks' gradient. A stream of 4·D bytes per row: a block
-// takes 32 tokens x 8 heads, D / 8 lanes per row with one 16-byte load of each operand, and turns
-// the sums in shared memory so that they leave as whole 128-byte lines along t. The sink gradient
-// is one atomic per (32 tokens, head): with one per row, all rows of a head queued on one address
-// (2 x 4096 x 64 heads of 64: 379 us, now 35; without sinks, 2 x 4096 x 32 heads of 128: 59 us, now 31).
-constexpr int DELTA_T = 32, DELTA_H = 8;
-template <int D>
+// takes TT tokens x 8 heads, D / 8 lanes per row with one 16-byte load of each operand, four rows' loads
+// in flight, and turns the sums in shared memory so that they leave as whole lines along t (128 bytes
+// with 32 tokens). The sink gradient is one atomic per (TT tokens, head): with one per row, all rows of a head
+// queued on one address (2 x 4096 x 64 heads of 64: 379 us, now 35; without sinks, 2 x 4096 x 32 heads of
+// 128: 59 us, now 31). Few rows take 8 tokens per block, one step for a thread: with 32, sixteen
+// of them waited for memory one after another (64 tokens of 32 heads of 128: 6.5 us, a warp per row 2.2).
+constexpr int DELTA_H = 8;
+template <int D, int TT>
 __global__ void __launch_bounds__(256)
 attn_delta_kernel(const __nv_bfloat16* __restrict__ o, const __nv_bfloat16* __restrict__ d_o,
                   const float* __restrict__ lse, const float* __restrict__ sinks,
                   float* __restrict__ delta, float* __restrict__ dsinks, int T, int H, bool o16) {
   constexpr int LPR = D / 8;            // lanes per row
   constexpr int PER = 256 / LPR;        // rows the block works on at once
-  __shared__ float sums[DELTA_H][DELTA_T + 1];
-  const int t0 = blockIdx.x * DELTA_T, h0 = blockIdx.y * DELTA_H, b = blockIdx.z;
+  constexpr int ROWS = TT * DELTA_H, FLY = ROWS / PER < 4 ? ROWS / PER : 4;
+  __shared__ float sums[DELTA_H][TT + 1];
+  const int t0 = blockIdx.x * TT, h0 = blockIdx.y * DELTA_H, b = blockIdx.z;
   const int li = threadIdx.x % LPR, first = threadIdx.x / LPR;
-#pragma unroll 4
-  for (int i = first; i < DELTA_T * DELTA_H; i += PER) {
-    const int t = t0 + i / DELTA_H, h = h0 + i % DELTA_H;
-    float acc = 0.f;
-    if (t < T && h < H) {
-      const size_t at = (((size_t)b * T + t) * H + h) * D + li * 8;
-      const uint4 y = *reinterpret_cast<const uint4*>(d_o + at);
-      uint4 x;
-      if (o16) {
-        x = *reinterpret_cast<const uint4*>(o + at);
-      } else {   // O starts between 16-byte boundaries (dO's start the tensor map checks)
-        const unsigned short* p = reinterpret_cast<const unsigned short*>(o + at);
-        x = make_uint4(p[0] | (uint32_t)p[1] << 16, p[2] | (uint32_t)p[3] << 16, p[4] | (uint32_t)p[5] << 16,
-                       p[6] | (uint32_t)p[7] << 16);
+#pragma unroll 1
+  for (int i0 = first; i0 < ROWS; i0 += FLY * PER) {
+    uint4 x[FLY], y[FLY];
+#pragma unroll
+    for (int f = 0; f < FLY; ++f) {
+      const int i = i0 + f * PER, t = t0 + i / DELTA_H, h = h0 + i % DELTA_H;
+      x[f] = y[f] = make_uint4(0, 0, 0, 0);
+      if (t < T && h < H) {
+        const size_t at = (((size_t)b * T + t) * H + h) * D + li * 8;
+        y[f] = *reinterpret_cast<const uint4*>(d_o + at);
+        if (o16) {
+          x[f] = *reinterpret_cast<const uint4*>(o + at);
+        } else {   // O starts between 16-byte boundaries (dO's start the tensor map checks)
+          const unsigned short* p = reinterpret_cast<const unsigned short*>(o + at);
+          x[f] = make_uint4(p[0] | (uint32_t)p[1] << 16, p[2] | (uint32_t)p[3] << 16, p[4] | (uint32_t)p[5] << 16,
+                            p[6] | (uint32_t)p[7] << 16);
+        }
       }
-      const uint32_t* xu = &x.x; const uint32_t* yu = &y.x;
+    }
+#pragma unroll
+    for (int f = 0; f < FLY; ++f) {
+      const uint32_t* xu = &x[f].x; const uint32_t* yu = &y[f].x;
+      float acc = 0.f;
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float2 p = unpack_bf16(xu[j]), g = unpack_bf16(yu[j]);
         acc += p.x * g.x + p.y * g.y;
       }
-    }
 #pragma unroll
-    for (int s = LPR / 2; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
-    if (li == 0) sums[i % DELTA_H][i / DELTA_H] = acc;
+      for (int s = LPR / 2; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+      const int i = i0 + f * PER;
+      if (li == 0) sums[i % DELTA_H][i / DELTA_H] = acc;
+    }
   }
   __syncthreads();
   const int t = t0 + (threadIdx.x & 31), h = h0 + (threadIdx.x >> 5);   // a warp per head
   if (h >= H) return;
   float ds = 0.f;
-  if (t < T) {
+  if (t < T && (threadIdx.x & 31) < TT) {
     const size_t idx = ((size_t)b * H + h) * T + t;
     const float acc = sums[threadIdx.x >> 5][threadIdx.x & 31];
     delta[idx] = acc;
@@ -527,9 +538,12 @@ static const char* attn_bwd_launch_d(const AttnArgs& a, cudaStream_t stream) {
   static bool configured[64] = {};
   if (!allow_dynamic_smem(kern, Cfg::SMEM_BYTES, configured))
     return "cudaFuncSetAttribute(max dynamic shared memory) failed";
-  attn_delta_kernel<D><<<dim3((a.T + DELTA_T - 1) / DELTA_T, (a.H + DELTA_H - 1) / DELTA_H, a.B), 256, 0, stream>>>(
-      reinterpret_cast<const __nv_bfloat16*>(a.o), reinterpret_cast<const __nv_bfloat16*>(a.d_o), a.lse,
-      a.sinks, a.delta, a.dsinks, a.T, a.H, reinterpret_cast<uintptr_t>(a.o) % 16 == 0);
+  const long tiles = (long)((a.T + 31) / 32) * ((a.H + DELTA_H - 1) / DELTA_H) * a.B;
+#define DELTA_CASE(TT_) attn_delta_kernel<D, TT_><<<dim3((a.T + TT_ - 1) / TT_, (a.H + DELTA_H - 1) / DELTA_H, a.B), 256, 0, stream>>>( \
+      reinterpret_cast<const __nv_bfloat16*>(a.o), reinterpret_cast<const __nv_bfloat16*>(a.d_o), a.lse, \
+      a.sinks, a.delta, a.dsinks, a.T, a.H, reinterpret_cast<uintptr_t>(a.o) % 16 == 0)
+  if (tiles < 148 * 4) DELTA_CASE(8); else DELTA_CASE(32);   // half of what is resident: fewer leave the GPU waiting
+#undef DELTA_CASE
   const long grid = (long)((a.S + BT - 1) / BT) * a.G * a.B;
   if (grid >= (1L << 31)) return "too many key tiles for one launch";
   kern<<<(unsigned)grid, BWD_THREADS, Cfg::SMEM_BYTES, stream>>>(p);
