@@ -95,30 +95,42 @@ rmsnorm_fwd_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict_
   }
 }
 
-// Rows wider than a warp holds (d / 8 threads per block, d <= 8192): a thread owns eight columns of
-// ROWS rows, loaded together; the squares meet in shared memory. 8192 x 4096: 55 us with a warp per
-// row, 38 so (two rows; with four, 8192 x 2880 takes 31 instead of 27).
-template <int THREADS, int ROWS>
-__global__ void __launch_bounds__(THREADS)
+// Rows wider than a warp holds (d <= 8192), and few rows of 1024 and more: a thread owns PIECES times eight
+// columns of ROWS rows, loaded together; the squares meet in shared memory. 8192 x 4096: 55 us with a
+// warp per row, 38 so (two rows; with four, 8192 x 2880 takes 31 instead of 27). Beyond 4096 columns two
+// pieces per thread keep two blocks on an SM, one loading while the other waits for its sums (32768 x 8192: a
+// warp per row 341 us, one block of 1024 threads 400, so 211; 32768 x 6144 257, 309, 174).
+template <int PIECES, int ROWS>
+__global__ void __launch_bounds__(512, PIECES > 1 ? 2 : 3)
 rmsnorm_fwd_columns_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w, bool w16,
                            __nv_bfloat16* __restrict__ y, float* __restrict__ rstd, int rows, int d, float eps) {
-  __shared__ float part[32][ROWS];
-  const int nvec = d / 8, i = threadIdx.x, nw = blockDim.x >> 5, r0 = blockIdx.x * ROWS;
-  const bool mine = i < nvec;
-  uint4 v[ROWS];
-#pragma unroll
-  for (int k = 0; k < ROWS; ++k)
-    v[k] = mine && r0 + k < rows ? reinterpret_cast<const uint4*>(x)[(size_t)(r0 + k) * nvec + i] : make_uint4(0, 0, 0, 0);
-  float g[8];
-  if (mine) load_gain8(w, w16, i, g);
+  __shared__ float part[16][ROWS];
+  const int nvec = d / 8, nw = blockDim.x >> 5, r0 = blockIdx.x * ROWS;
+  uint4 v[ROWS][PIECES];
 #pragma unroll
   for (int k = 0; k < ROWS; ++k) {
-    float f[8], ss = 0.f;
-    unpack8(v[k], f);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+    for (int p = 0; p < PIECES; ++p) {
+      const int i = threadIdx.x + p * blockDim.x;
+      v[k][p] = i < nvec && r0 + k < rows ? reinterpret_cast<const uint4*>(x)[(size_t)(r0 + k) * nvec + i] : make_uint4(0, 0, 0, 0);
+    }
+  }
+  float g[PIECES][8];
+#pragma unroll
+  for (int p = 0; p < PIECES; ++p)
+    if (threadIdx.x + p * blockDim.x < nvec) load_gain8(w, w16, threadIdx.x + p * blockDim.x, g[p]);
+#pragma unroll
+  for (int k = 0; k < ROWS; ++k) {
+    float ss = 0.f;
+#pragma unroll
+    for (int p = 0; p < PIECES; ++p) {
+      float f[8];
+      unpack8(v[k][p], f);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) ss += f[j] * f[j];
+    }
     ss = warp_sum(ss);
-    if ((i & 31) == 0) part[i >> 5][k] = ss;
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5][k] = ss;
   }
   __syncthreads();
 #pragma unroll
@@ -127,13 +139,17 @@ rmsnorm_fwd_columns_kernel(const __nv_bfloat16* __restrict__ x, const float* __r
     for (int q = 0; q < nw; ++q) ss += part[q][k];
     const float r = rsqrtf(ss / d + eps);
     if (r0 + k >= rows) break;
-    if (i == 0 && rstd) rstd[r0 + k] = r;
-    float f[8];
-    unpack8(v[k], f);
-    if (mine) {
+    if (threadIdx.x == 0 && rstd) rstd[r0 + k] = r;
 #pragma unroll
-      for (int j = 0; j < 8; ++j) f[j] = f[j] * r * g[j];
-      reinterpret_cast<uint4*>(y)[(size_t)(r0 + k) * nvec + i] = pack8(f);
+    for (int p = 0; p < PIECES; ++p) {
+      const int i = threadIdx.x + p * blockDim.x;
+      float f[8];
+      unpack8(v[k][p], f);
+      if (i < nvec) {
+#pragma unroll
+        for (int j = 0; j < 8; ++j) f[j] = f[j] * r * g[p][j];
+        reinterpret_cast<uint4*>(y)[(size_t)(r0 + k) * nvec + i] = pack8(f);
+      }
     }
   }
 }
@@ -1538,13 +1554,16 @@ void rmsnorm_fwd(const void* x, const float* w, void* y, float* rstd, long rows,
   const int nv = threads / 32;   // 16-byte pieces of a row per lane; 8 of them are the most held
 #define RN_CASE(NV_, COND) \
   if (COND) { rmsnorm_fwd_kernel<NV_><<<grid, wpb * 32, 0, s>>>((const __nv_bfloat16*)x, w, w16, (__nv_bfloat16*)y, rstd, (int)rows, d, eps); return; }
-  RN_CASE(1, nv <= 1) RN_CASE(2, nv <= 2) RN_CASE(4, nv <= 4) RN_CASE(8, nv <= 8)
-#define RC_CASE(THREADS_, ROWS_) \
-  if (threads <= THREADS_) { \
-    rmsnorm_fwd_columns_kernel<THREADS_, ROWS_><<<(int)((rows + ROWS_ - 1) / ROWS_), threads, 0, s>>>( \
+#define RC_CASE(PIECES_, ROWS_, COND) \
+  if (COND) { \
+    rmsnorm_fwd_columns_kernel<PIECES_, ROWS_><<<(int)((rows + ROWS_ - 1) / ROWS_), PIECES_ == 1 ? threads : (threads / 2 + 31) / 32 * 32, 0, s>>>( \
         (const __nv_bfloat16*)x, w, w16, (__nv_bfloat16*)y, rstd, (int)rows, d, eps); \
     return; }
-  RC_CASE(512, 2) RC_CASE(1024, 2)
+  // few rows: a block each, so that a lane waits for one load and not for eight (300 x 2048 2.3 us, a warp
+  // per row 4.2; at 1000 rows 4.4 either way)
+  RC_CASE(1, 1, rows <= 592 && nv > 2 && nv <= 8)
+  RN_CASE(1, nv <= 1) RN_CASE(2, nv <= 2) RN_CASE(4, nv <= 4) RN_CASE(8, nv <= 8)
+  RC_CASE(1, 2, threads <= 512) RC_CASE(2, 2, threads <= 1024)
 #undef RC_CASE
   RN_CASE(0, true)
 #undef RN_CASE

@@ -202,7 +202,8 @@ def test_rmsnorm(cuda):
     assert rel_err(dw, w.grad) < 2e-2
 
 
-@pytest.mark.parametrize("rows,d", [(1, 8), (5, 504), (3, 512), (9, 1032), (2, 2056), (5, 2880), (3, 4104), (2, 8192), (3, 8200)])
+@pytest.mark.parametrize("rows,d", [(1, 8), (5, 504), (3, 512), (9, 1032), (2, 2056), (5, 2880), (3, 4104), (2, 8192), (3, 8200),
+                                    (592, 520), (593, 520), (601, 1032), (593, 2048), (601, 4104)])
 @pytest.mark.parametrize("shift", [0, 1])
 def test_rmsnorm_widths(cuda, rows, d, shift):
     """The edges of each way of splitting a row, and gains that start between 16-byte boundaries.
