@@ -302,7 +302,7 @@ __global__ void rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const fl
 // its columns of the slab, so the per-row update is a plain vector read-modify-write (no
 // atomics); the slabs are summed once at the end. Needs 8 warps · d · 4 bytes of shared memory.
 __global__ void __launch_bounds__(256)
-rmsnorm_bwd_slab_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w, bool w16,
+rmsnorm_bwd_slab_kernel(const __nv_bfloat16* __restrict__ x, const float* __restrict__ w,
                         const __nv_bfloat16* __restrict__ dy, const float* __restrict__ rstd,
                         __nv_bfloat16* __restrict__ dx, float* __restrict__ dw, int rows, int d) {
   extern __shared__ __align__(16) float slabs[];  // [warps][d]
@@ -311,6 +311,7 @@ rmsnorm_bwd_slab_kernel(const __nv_bfloat16* __restrict__ x, const float* __rest
   for (int i = threadIdx.x; i < warps_per_block * d; i += blockDim.x) slabs[i] = 0.f;
   __syncthreads();
   float4* mine = reinterpret_cast<float4*>(slabs + (size_t)warp * d);
+  const float4* w4 = reinterpret_cast<const float4*>(w);
   const int nvec = d / 8;
   for (int row = blockIdx.x * warps_per_block + warp; row < rows; row += gridDim.x * warps_per_block) {
     const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)row * d);
@@ -320,8 +321,11 @@ rmsnorm_bwd_slab_kernel(const __nv_bfloat16* __restrict__ x, const float* __rest
     for (int i = lane; i < nvec; i += 32) {
       const uint4 xv = xr[i], gv = gr[i];
       const uint32_t* xu = &xv.x; const uint32_t* gu = &gv.x;
-      float wl[8];
-      load_gain8(w, w16, i, wl);
+      float wl[8] = {1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f};
+      if (w) {
+        const float4 lo = w4[2 * i], hi = w4[2 * i + 1];
+        wl[0] = lo.x; wl[1] = lo.y; wl[2] = lo.z; wl[3] = lo.w; wl[4] = hi.x; wl[5] = hi.y; wl[6] = hi.z; wl[7] = hi.w;
+      }
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         const float2 a = unpack_bf16(xu[j]), g = unpack_bf16(gu[j]);
@@ -334,8 +338,11 @@ rmsnorm_bwd_slab_kernel(const __nv_bfloat16* __restrict__ x, const float* __rest
     for (int i = lane; i < nvec; i += 32) {
       const uint4 xv = xr[i], gv = gr[i];  // second read of the row: L1 / L2
       const uint32_t* xu = &xv.x; const uint32_t* gu = &gv.x;
-      float wl[8];
-      load_gain8(w, w16, i, wl);
+      float wl[8] = {1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f, 1.f};
+      if (w) {
+        const float4 lo = w4[2 * i], hi = w4[2 * i + 1];
+        wl[0] = lo.x; wl[1] = lo.y; wl[2] = lo.z; wl[3] = lo.w; wl[4] = hi.x; wl[5] = hi.y; wl[6] = hi.z; wl[7] = hi.w;
+      }
       uint4 o; uint32_t* ou = &o.x;
       float p[8];
 #pragma unroll
@@ -1595,8 +1602,8 @@ void rmsnorm_bwd(const void* x, const float* w, const void* dy, const float* rst
   }
   const int wpb = 8;
   int grid = (int)min((rows + wpb - 1) / wpb, 148L * 4);
-  if (d % 8 == 0 && d < 512) {
-    rmsnorm_bwd_slab_kernel<<<grid, wpb * 32, (size_t)wpb * d * sizeof(float), s>>>((const __nv_bfloat16*)x, w, w16, (const __nv_bfloat16*)dy, rstd, (__nv_bfloat16*)dx, dw, (int)rows, d);
+  if (d % 8 == 0 && d < 512 && w16) {   // gains between 16-byte boundaries: the kernel below
+    rmsnorm_bwd_slab_kernel<<<grid, wpb * 32, (size_t)wpb * d * sizeof(float), s>>>((const __nv_bfloat16*)x, w, (const __nv_bfloat16*)dy, rstd, (__nv_bfloat16*)dx, dw, (int)rows, d);
     return;
   }
   rmsnorm_bwd_kernel<<<grid, wpb * 32, d * sizeof(float), s>>>(
