@@ -223,9 +223,10 @@ def test_rmsnorm_widths(cuda, rows, d, shift):
     assert rel_err(plain, want / wd) < 4e-3 and rel_err(K.rmsnorm_bwd(x, None, dy, r2)[0], K.rmsnorm_bwd(x, torch.ones_like(w), dy, r2)[0]) < 1e-6
 
 
-@pytest.mark.parametrize("tokens,heads,d", [(1, 1, 64), (7, 3, 128), (33, 5, 256), (50, 6, 64)])
+@pytest.mark.parametrize("tokens,heads,d", [(1, 1, 64), (7, 3, 128), (33, 5, 256), (50, 6, 64),
+                                            (5000, 1, 128), (1600, 7, 64), (700, 5, 256), (1000, 6, 128)])
 def test_norm_rope_odd_heads(cuda, tokens, heads, d):
-    """Heads go four (backward: two) at a time: counts that they do not divide, and a slice of wider
+    """Heads go four (backward: two) at a time, few of them one by one: counts that they do not divide, and a slice of wider
     rows. Bounds as for the RMSNorm, with one rotation more."""
     from bux_b200.ops import kernels as K
 
