@@ -1016,8 +1016,9 @@ __global__ void quant_nvfp4_kernel(const __nv_bfloat16* __restrict__ x, const fl
 // is rescaled only when its maximum moves), then the gradient; the second walk finds most of the row
 // in L2. Four 16-byte loads per thread in flight and three blocks per SM: 4096 x 151936 took 840 us
 // with separate walks for the maximum and the sum, 576 now (597 at two blocks; one read and one
-// write of device memory would take 381).
-constexpr int CE_THREADS = 512, CE_BLOCKS = 3, CE_UNROLL = 4;
+// write of device memory would take 381). Rows that do not give 512 threads a load each take 128, and many
+// rows of up to 4096 entries 256 (2048 x 128: 4.3 us, 10.1 with 512; 2048 x 4096: 12.5 and 16.7).
+constexpr int CE_UNROLL = 4;
 __device__ __forceinline__ void ce_load8(const uint4& v, float softcap, float (&t)[8]) {
   unpack8(v, t);
   if (softcap > 0.f) {
@@ -1025,7 +1026,8 @@ __device__ __forceinline__ void ce_load8(const uint4& v, float softcap, float (&
     for (int j = 0; j < 8; ++j) t[j] = softcap * tanhf(t[j] / softcap);
   }
 }
-__global__ void __launch_bounds__(CE_THREADS, CE_BLOCKS)
+template <int CE_THREADS>
+__global__ void __launch_bounds__(CE_THREADS, 1536 / CE_THREADS)
 ce_fwd_bwd_kernel(__nv_bfloat16* __restrict__ logits, const int* __restrict__ targets,
                   const float* __restrict__ mask, float* __restrict__ loss,
                   float* __restrict__ logz_out, int vocab, long ld, float grad_scale,
@@ -1679,7 +1681,9 @@ void quant_nvfp4(const void* x, const float* tensor_scale, uint8_t* packed, uint
   quant_nvfp4_kernel<<<grid_for(blocks, 256), 256, 0, s>>>((const __nv_bfloat16*)x, tensor_scale, packed, scales, blocks);
 }
 void ce_fwd_bwd(void* logits, const int* targets, const float* mask, float* loss, float* logz, long rows, int vocab, long ld, float grad_scale, float z_weight, float softcap, cudaStream_t s) {
-  ce_fwd_bwd_kernel<<<(unsigned)rows, CE_THREADS, 0, s>>>((__nv_bfloat16*)logits, targets, mask, loss, logz, vocab, ld, grad_scale, z_weight, softcap);
+#define CE_CASE(THREADS_) ce_fwd_bwd_kernel<THREADS_><<<(unsigned)rows, THREADS_, 0, s>>>((__nv_bfloat16*)logits, targets, mask, loss, logz, vocab, ld, grad_scale, z_weight, softcap)
+  if (vocab <= 8 * 128) CE_CASE(128); else if (vocab <= 8 * 512 && rows > 148 * 4) CE_CASE(256); else CE_CASE(512);
+#undef CE_CASE
 }
 void scale_to_bf16(const void* src, bool src_bf16, const float* scale, void* out, long n, cudaStream_t s) {
   const int grid = grid_for(n / 8, 256 * 4, 148 * 8);

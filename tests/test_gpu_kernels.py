@@ -350,16 +350,17 @@ def test_cross_entropy(cuda):
     assert rel_err(work, lf.grad) < 2e-2
 
 
-@pytest.mark.parametrize("vocab", [8, 4096, 16384 + 8, 50304])
+@pytest.mark.parametrize("vocab,rows", [(8, 5), (1024, 5), (1032, 5), (4096, 5), (1032, 593), (4096, 600), (4104, 600),
+                                        (16384 + 8, 5), (50304, 5)])
 @pytest.mark.parametrize("case", ["plain", "masked", "softcap"])
-def test_cross_entropy_rows_and_masked_logits(cuda, vocab, case):
-    """One pass keeps the maximum and the sum: rows shorter than a block's step, remainders of the
-    unrolled walk, logits of -inf and of the type's lowest value, a maximum that comes last.
+def test_cross_entropy_rows_and_masked_logits(cuda, vocab, rows, case):
+    """One pass keeps the maximum and the sum: the three widths of a block, rows shorter than its step,
+    remainders of the unrolled walk, logits of -inf and of the type's lowest value, a maximum that comes last.
     Bounds: the loss is an fp32 sum, the gradient is rounded to bf16 (2^-9)."""
     from bux_b200.ops import kernels as K
 
     torch.manual_seed(8)
-    rows, cap = 5, 20.0 if case == "softcap" else 0.0
+    cap = 20.0 if case == "softcap" else 0.0
     logits = (torch.randn(rows, vocab, device=cuda) * 4).bfloat16()
     targets = torch.randint(0, vocab, (rows,), device=cuda, dtype=torch.int32)
     logits[1, -1] = 60.0
