@@ -454,6 +454,12 @@ static const char* attn_fwd_launch_d(const AttnArgs& a, cudaStream_t stream) {
   static bool configured[64] = {};
   if (!allow_dynamic_smem(kern, Cfg::SMEM_BYTES, configured))
     return "cudaFuncSetAttribute(max dynamic shared memory) failed";
+  // the register split counts on what the compiler gave the block; with less its increase would wait for ever
+  static const bool enough = [&] {
+    cudaFuncAttributes attr;
+    return cudaFuncGetAttributes(&attr, kern) == cudaSuccess && attr.numRegs >= FWD_LAUNCH_REGS;
+  }();
+  if (!enough) return "the attention kernel was compiled with fewer registers than its split hands out";
   const long grid = (long)((a.T + 2 * QT - 1) / (2 * QT)) * a.H * a.B;
   if (grid >= (1L << 31)) return "too many query tiles for one launch";
   kern<<<(unsigned)grid, FWD_THREADS, Cfg::SMEM_BYTES, stream>>>(p);
