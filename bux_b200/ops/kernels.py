@@ -98,12 +98,29 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: boo
     return out
 
 
-def _tile_width(n: int, kind: int) -> int:
-    """256-wide tiles halve the operand traffic per FLOP: taken when they tile N exactly, and in bf16
-    (whose operands need no whole scale tiles) where they cover at most a quarter more columns than
-    narrow ones (32 experts of 5760 x 2880, 128 rows each: 233 us wide, 282 narrow, 4 % more columns)."""
-    wide, narrow = -(-n // 256) * 256, -(-n // 128) * 128
-    return 256 if n % 256 == 0 or (kind == KIND_BF16 and wide * 4 <= narrow * 5) else 128
+_SMS = 148  # SMs of the chip
+
+
+def _tile_width(n: int, kind: int, row_tiles: float, margin: float = 1.0) -> int:
+    """Columns per tile of a grouped product of `n` columns and about `row_tiles` tiles of 128 rows.
+    256-wide tiles halve the operand traffic per FLOP: taken when they tile N exactly. In bf16 (whose
+    operands need no whole scale tiles) also where they cover at most a quarter more columns than
+    narrow ones and, a wave of narrow tiles costing 0.62 of one of wide ones (see `gemm_plan`), take no
+    longer by `margin`: 32 experts of 5760 x 2880, 128 rows each 233 us wide, 282 narrow; 4 x 2880 x 2880 with 100
+    rows each 33 wide, 27 narrow; 16 x 896 x 2048 with 256 rows each 50 and 38, with 512 51 and 56."""
+    wide, narrow = -(-n // 256), -(-n // 128)
+    if n % 256 == 0:
+        return 256
+    if kind != KIND_BF16 or wide * 2 * 4 > narrow * 5:
+        return 128
+    return 256 if -(-row_tiles * narrow // _SMS) * 0.62 >= margin * -(-row_tiles * wide // _SMS) else 128
+
+
+def _grouped_row_tiles(rows: int, groups: int) -> float:
+    """Tiles of 128 rows that `rows` sorted rows are likely to have: without each group's padding, half
+    a tile per group more than they fill, and one per group that has a row."""
+    live = max(1, rows - 127 * groups)
+    return max(min(groups, live), live / 128 + groups / 2)
 
 
 def gemm_mxfp8(aq, asf, bq, bsf, m: int, n: int, k: int, *, out=None, out_dtype=torch.bfloat16,
@@ -124,8 +141,9 @@ def grouped_gemm(a, b, offsets: torch.Tensor, n: int, k: int, *, kind: int = KIN
                  wait_flags=None, wait_epoch: int = 0) -> torch.Tensor:
     """Rows of `a` ([R,k], sorted by group; offsets int32[G+1]) times group g's weight.
     b: [G*n, k] (K-major) or [G*k, n] (b_mn). Returns [R, n] bf16."""
-    bn = _tile_width(n, kind) if bn is None else bn
     groups = offsets.numel() - 1
+    # (a product of few rows streams its weights: the wide tile has to win by a little)
+    bn = _tile_width(n, kind, _grouped_row_tiles(a.shape[0], groups), 1.05) if bn is None else bn
     if out is None:
         out = _out(a.shape[0], n, dtype=torch.bfloat16, device=a.device, op="grouped_gemm")
     if kind == KIND_MXFP8:
@@ -144,8 +162,8 @@ def grouped_gemm_k(a, b, offsets: torch.Tensor, m: int, n: int, *, kind: int = K
     gradients of grouped experts). K-major: a [m, Ktot], b [n, Ktot]; MN-major: a [Ktot, m],
     b [Ktot, n]. Returns [G, m, n] in `out_dtype` (fp32, or bf16 written straight from the
     accumulator when that is what the gradient is kept in)."""
-    bn = _tile_width(n, kind) if bn is None else bn
     groups = offsets.numel() - 1
+    bn = _tile_width(n, kind, groups * -(-m // 128)) if bn is None else bn
     ktot = a.shape[0] if a_mn else a.shape[1]
     if out is None:
         out = _out(groups, m, n, dtype=out_dtype, device=a.device, op="grouped_gemm_k")

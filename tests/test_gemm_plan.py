@@ -40,3 +40,19 @@ def test_pairs_of_sms_take_what_fills_them(m, n, k, pairs):
 def test_short_contractions_are_not_split(kind, m, n, k, splits):
     """The ranges have to save more than the second launch and the partial sums cost."""
     assert K.ops().gemm_plan(kind, m, n, k)[1] == splits
+
+
+@pytest.mark.parametrize("groups,rows_each,n,width", [
+    (4, 75, 2880, 128), (4, 194, 2880, 256), (16, 256, 896, 128), (16, 512, 896, 256), (8, 40, 640, 128),
+    (32, 97, 2880, 256), (32, 16, 2880, 128), (32, 97, 5760, 256), (8, 4, 4992, 128), (8, 512, 4992, 256),
+    (8, 512, 384, 128), (8, 4, 512, 256)])
+def test_ragged_widths_of_grouped_products(groups, rows_each, n, width):
+    """Widths that 256 does not divide take the tile whose waves are shorter; measured either way."""
+    rows = groups * (rows_each + 127)
+    assert K._tile_width(n, K.KIND_BF16, K._grouped_row_tiles(rows, groups), 1.05) == width
+    assert K._tile_width(n, K.KIND_MXFP8, K._grouped_row_tiles(rows, groups), 1.05) == (256 if n % 256 == 0 else 128)
+
+
+@pytest.mark.parametrize("groups,m,n,width", [(32, 2880, 2880, 256), (128, 2048, 640, 256), (8, 384, 640, 128), (16, 2048, 896, 256)])
+def test_ragged_widths_of_grouped_weight_gradients(groups, m, n, width):
+    assert K._tile_width(n, K.KIND_BF16, groups * -(-m // 128)) == width
