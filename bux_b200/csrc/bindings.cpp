@@ -40,6 +40,13 @@ const int* opt_i32(const c10::optional<Tensor>& t) {
   return t->data_ptr<int>();
 }
 
+// Workspace a kernel writes: the caller's (kernel checks put it between guards) or a new one.
+Tensor scratch_f32(const c10::optional<Tensor>& given, at::IntArrayRef shape, const Tensor& like) {
+  if (!given.has_value()) return at::empty(shape, like.options().dtype(at::kFloat));
+  TORCH_CHECK(given->is_cuda() && given->scalar_type() == at::kFloat && given->is_contiguous() && given->sizes() == shape, "scratch: fp32 ", shape);
+  return *given;
+}
+
 // ------------------------------------------------------------------ GEMM
 // c (+)= a · b^T.  kind 0 = bf16, 1 = mxfp8 (a/b uint8 e4m3 bytes, sfa/sfb tiled scales).
 // a_mn / b_mn: operand stored transposed ([K, M] / [K, N]).  mode: 0 dense, 1 grouped rows
@@ -49,7 +56,7 @@ void gemm(const Tensor& a, const Tensor& b, Tensor& c, const c10::optional<Tenso
           const c10::optional<Tensor>& status, int64_t kind, int64_t mode, int64_t M, int64_t N,
           int64_t K, int64_t k_total, int64_t groups, bool a_mn, bool b_mn, int64_t out_kind,
           int64_t bn, int64_t sms, const c10::optional<Tensor>& wait_flags, int64_t wait_epoch,
-          int64_t wait_rows, int64_t m_rotate, bool wait_on_k, bool wait_on_n) {
+          int64_t wait_rows, int64_t m_rotate, bool wait_on_k, bool wait_on_n, const c10::optional<Tensor>& scratch) {
   check_cuda(a, "a"); check_cuda(b, "b"); check_cuda(c, "c");
   TORCH_CHECK(a.dim() == 2 && b.dim() == 2, "a and b are 2-D views");
   c10::cuda::CUDAGuard guard(a.device());
@@ -86,7 +93,7 @@ void gemm(const Tensor& a, const Tensor& b, Tensor& c, const c10::optional<Tenso
     const bux::GemmPlan plan = bux::gemm_plan(g.kind, M, N, K, g.sms, may_split);
     g.bn = plan.bn;
     if (plan.splits > 1) {
-      partial = at::empty({plan.splits, M, N}, c.options().dtype(at::kFloat));
+      partial = scratch_f32(scratch, {plan.splits, M, N}, c);
       g.splits = plan.splits; g.partial = partial.data_ptr<float>();
     }
   }
@@ -94,9 +101,9 @@ void gemm(const Tensor& a, const Tensor& b, Tensor& c, const c10::optional<Tenso
   TORCH_CHECK(err == nullptr, "bux gemm: ", err);
 }
 
-std::vector<int64_t> gemm_plan(int64_t kind, int64_t M, int64_t N, int64_t K) {
-  const bux::GemmPlan plan = bux::gemm_plan((int)kind, M, N, K, 0, true);
-  return {plan.bn, plan.splits, kind == bux::KIND_BF16 && plan.bn == 256 && plan.splits == 1 && bux::gemm_pairs(M, N, K)};
+std::vector<int64_t> gemm_plan(int64_t kind, int64_t M, int64_t N, int64_t K, int64_t sms) {
+  const bux::GemmPlan plan = bux::gemm_plan((int)kind, M, N, K, (int)sms, true);
+  return {plan.bn, plan.splits, sms <= 0 && kind == bux::KIND_BF16 && plan.bn == 256 && plan.splits == 1 && bux::gemm_pairs(M, N, K)};
 }
 
 // ------------------------------------------------------------------ norms
@@ -108,7 +115,7 @@ void rmsnorm_fwd(const Tensor& x, const c10::optional<Tensor>& w, Tensor& y, Ten
   bux::rmsnorm_fwd(x.data_ptr(), opt_f32(w), y.data_ptr(), rstd.data_ptr<float>(), x.numel() / d, d, (float)eps, stream_of(x));
 }
 void rmsnorm_bwd(const Tensor& x, const c10::optional<Tensor>& w, const Tensor& dy, const Tensor& rstd,
-                 Tensor& dx, const c10::optional<Tensor>& dw) {
+                 Tensor& dx, const c10::optional<Tensor>& dw, const c10::optional<Tensor>& scratch) {
   check_cuda(x, "x"); check_cuda(dy, "dy"); check_cuda(dx, "dx");
   const int d = (int)x.size(-1);
   TORCH_CHECK(d > 0, "rmsnorm: rows of at least one element");
@@ -117,7 +124,7 @@ void rmsnorm_bwd(const Tensor& x, const c10::optional<Tensor>& w, const Tensor& 
   Tensor part;
   if (dwp) {
     const int n = bux::rmsnorm_bwd_partials(x.numel() / d, d);
-    if (n > 0) part = at::empty({n, d}, dw->options());
+    if (n > 0) part = scratch_f32(scratch, {n, d}, *dw);
     else dw->zero_();
   }
   bux::rmsnorm_bwd(x.data_ptr(), opt_f32(w), dy.data_ptr(), rstd.data_ptr<float>(), dx.data_ptr(), dwp,
@@ -290,7 +297,7 @@ void topk_rows(const Tensor& scores, Tensor& idx) {
   TORCH_CHECK(err == nullptr, err);
 }
 void sort_picks(const Tensor& experts, const c10::optional<Tensor>& weights, Tensor& row_index, Tensor& pos, Tensor& offsets,
-                const c10::optional<Tensor>& w_row, const c10::optional<Tensor>& status, int64_t align) {
+                const c10::optional<Tensor>& w_row, const c10::optional<Tensor>& status, int64_t align, const c10::optional<Tensor>& scratch) {
   check_cuda(experts, "experts"); check_cuda(row_index, "row_index"); check_cuda(pos, "pos"); check_cuda(offsets, "offsets");
   const int64_t n = experts.numel(), E = offsets.numel() - 1, rows = row_index.numel();
   TORCH_CHECK(experts.scalar_type() == at::kLong && experts.dim() == 2 && n > 0 && n < (1LL << 31), "sort_picks: int64 [t, k]");
@@ -302,7 +309,10 @@ void sort_picks(const Tensor& experts, const c10::optional<Tensor>& weights, Ten
   TORCH_CHECK(!weights.has_value() || weights->numel() == n, "sort_picks: a weight per pick");
   TORCH_CHECK(!w_row.has_value() || (w_row->scalar_type() == at::kFloat && w_row->numel() == rows && w_row->is_contiguous()), "sort_picks: w_row is fp32 [rows]");
   c10::cuda::CUDAGuard guard(experts.device());
-  Tensor work = at::empty({(bux::pick_blocks(n) + 1) * E}, offsets.options());
+  const int64_t words = (bux::pick_blocks(n) + 1) * E;
+  TORCH_CHECK(!scratch.has_value() || (scratch->is_cuda() && scratch->scalar_type() == at::kInt && scratch->is_contiguous() && scratch->numel() == words),
+              "sort_picks: scratch is int32 [", words, "]");
+  Tensor work = scratch.has_value() ? *scratch : at::empty({words}, offsets.options());
   bux::sort_picks(reinterpret_cast<const long long*>(experts.data_ptr<int64_t>()), opt_f32(weights), n, (int)experts.size(1), (int)E, (int)align,
                   row_index.data_ptr<int>(), pos.data_ptr<int>(), offsets.data_ptr<int>(), w_row.has_value() ? w_row->data_ptr<float>() : nullptr,
                   rows, work.data_ptr<int>(), status_ptr(status), stream_of(experts));
@@ -582,23 +592,25 @@ TORCH_LIBRARY(bux_b200, m) {
   m.def("sf_rows_to_tiles(Tensor src, Tensor(a!) dst) -> ()", &sf_rows_to_tiles);
   m.def("tp_push_block(Tensor src, Tensor peer_base, int my_rank, int sms) -> ()", &tp_push_block);
   m.def("tp_pull_reduce(Tensor peer_base, int my_rank, Tensor(a!) out, Tensor? residual, Tensor? flags, int epoch, Tensor? status, float limit_s) -> ()", &tp_pull_reduce);
-  m.def("gemm(Tensor a, Tensor b, Tensor(a!) c, Tensor? sfa, Tensor? sfb, Tensor? group_offsets, Tensor? status, int kind, int mode, int M, int N, int K, int k_total, int groups, bool a_mn, bool b_mn, int out_kind, int bn, int sms, Tensor? wait_flags=None, int wait_epoch=0, int wait_rows=0, int m_rotate=0, bool wait_on_k=False, bool wait_on_n=False) -> ()", &gemm);
+  m.def("gemm(Tensor a, Tensor b, Tensor(a!) c, Tensor? sfa, Tensor? sfb, Tensor? group_offsets, Tensor? status, int kind, int mode, int M, int N, int K, int k_total, int groups, bool a_mn, bool b_mn, int out_kind, int bn, int sms, Tensor? wait_flags=None, int wait_epoch=0, int wait_rows=0, int m_rotate=0, bool wait_on_k=False, bool wait_on_n=False, Tensor(b!)? scratch=None) -> ()", &gemm);
   m.def("rmsnorm_fwd(Tensor x, Tensor? w, Tensor(a!) y, Tensor(b!) rstd, float eps) -> ()", &rmsnorm_fwd);
-  m.def("rmsnorm_bwd(Tensor x, Tensor? w, Tensor dy, Tensor rstd, Tensor(a!) dx, Tensor? dw) -> ()", &rmsnorm_bwd);
+  m.def("rmsnorm_bwd(Tensor x, Tensor? w, Tensor dy, Tensor rstd, Tensor(a!) dx, Tensor? dw, Tensor(b!)? scratch=None) -> ()", &rmsnorm_bwd);
   m.def("norm_rope(bool bwd, Tensor x, Tensor? w, Tensor cos, Tensor sin, Tensor(a!) y, Tensor? rstd, Tensor? dy, Tensor? dw, int tokens, int heads, int D, int stride_x, int stride_y, float eps) -> ()", &norm_rope);
   m.def("glu_fwd(Tensor h, Tensor(a!) out, Tensor? row_scale, int kind, float limit, float up_offset) -> ()", &glu_fwd);
   m.def("glu_bwd(Tensor h, Tensor dout, Tensor(a!) dh, Tensor? row_scale, Tensor? d_row_scale, int kind, float limit, float up_offset) -> ()", &glu_bwd);
   m.def("quant_mxfp8(Tensor x, Tensor? row_index, Tensor? row_scale, Tensor? q_row, Tensor? sf_row, Tensor? q_col, Tensor? sf_col, int rows, int cols, int ld_col, int batch, int x_batch_stride) -> ()", &quant_mxfp8);
   m.def("quant_mxfp8_glu(Tensor h, Tensor? dout, Tensor? row_scale, Tensor? q_row, Tensor? sf_row, Tensor? q_col, Tensor? sf_col, int ld_col, int kind, float limit, float up_offset) -> ()", &quant_mxfp8_glu);
   m.def("quant_nvfp4(Tensor x, Tensor tensor_scale, Tensor(a!) packed, Tensor(b!) scales) -> ()", &quant_nvfp4);
-  m.def("gemm_plan(int kind, int M, int N, int K) -> int[]", &gemm_plan);
+  m.def("gemm_plan(int kind, int M, int N, int K, int sms=0) -> int[]", &gemm_plan);
+  m.def("rmsnorm_bwd_partials(int rows, int d) -> int", [](int64_t rows, int64_t d) { return (int64_t)bux::rmsnorm_bwd_partials(rows, (int)d); });
+  m.def("pick_blocks(int n) -> int", [](int64_t n) { return (int64_t)bux::pick_blocks(n); });
   m.def("token_stride(Tensor x) -> int", &token_stride);
   m.def("scale_to_bf16(Tensor src, Tensor scale, Tensor(a!) out) -> ()", &scale_to_bf16);
   m.def("ce_fwd_bwd(Tensor(a!) logits, Tensor targets, Tensor? mask, Tensor(b!) loss, Tensor? logz, float grad_scale, float z_weight, float softcap) -> ()", &ce_fwd_bwd);
   m.def("adamw(Tensor(a!) p, Tensor g, Tensor(b!) m, Tensor(c!) v, Tensor? m_sf, Tensor? v_sf, Tensor? shadow, Tensor? grad_scale, float lr, float b1, float b2, float eps, float wd, float bc1, float bc2, float grad_scale_const) -> ()", &adamw);
   m.def("sumsq(Tensor g, Tensor(a!) out) -> ()", &sumsq);
   m.def("topk_rows(Tensor scores, Tensor(a!) idx) -> ()", &topk_rows);
-  m.def("sort_picks(Tensor experts, Tensor? weights, Tensor(a!) row_index, Tensor(b!) pos, Tensor(c!) offsets, Tensor(d!)? w_row, Tensor(e!)? status, int align) -> ()", &sort_picks);
+  m.def("sort_picks(Tensor experts, Tensor? weights, Tensor(a!) row_index, Tensor(b!) pos, Tensor(c!) offsets, Tensor(d!)? w_row, Tensor(e!)? status, int align, Tensor(f!)? scratch=None) -> ()", &sort_picks);
   m.def("gather_rows(Tensor x, Tensor index, Tensor(a!) out) -> ()", &gather_rows);
   m.def("combine_bwd(Tensor? y, Tensor dout, Tensor pos, Tensor? w, Tensor(a!)? dy, Tensor(b!)? dw) -> ()", &combine_bwd);
   m.def("combine_rows(Tensor y, Tensor pos, Tensor? w, Tensor(a!) out) -> ()", &combine_rows);

@@ -9,9 +9,11 @@ using at::Tensor;
 void gemm(const Tensor& a, const Tensor& b, Tensor& c, const std::optional<Tensor>& sfa, const std::optional<Tensor>& sfb,
           const std::optional<Tensor>& group_offsets, const std::optional<Tensor>& status, int64_t kind, int64_t mode, int64_t M,
           int64_t N, int64_t K, int64_t k_total, int64_t groups, bool a_mn, bool b_mn, int64_t out_kind, int64_t bn, int64_t sms,
-          const std::optional<Tensor>& wait_flags, int64_t wait_epoch, int64_t wait_rows, int64_t m_rotate, bool wait_on_k, bool wait_on_n);
+          const std::optional<Tensor>& wait_flags, int64_t wait_epoch, int64_t wait_rows, int64_t m_rotate, bool wait_on_k, bool wait_on_n,
+          const std::optional<Tensor>& scratch = std::nullopt);
 void rmsnorm_fwd(const Tensor& x, const std::optional<Tensor>& w, Tensor& y, Tensor& rstd, double eps);
-void rmsnorm_bwd(const Tensor& x, const std::optional<Tensor>& w, const Tensor& dy, const Tensor& rstd, Tensor& dx, const std::optional<Tensor>& dw);
+void rmsnorm_bwd(const Tensor& x, const std::optional<Tensor>& w, const Tensor& dy, const Tensor& rstd, Tensor& dx, const std::optional<Tensor>& dw,
+                 const std::optional<Tensor>& scratch = std::nullopt);
 // Elements between tokens of x [..., T, H, D] when heads are dense and the leading dimensions collapse
 // into one (a column slice of a fused projection), x starts on 16 bytes and every token too; else -1.
 int64_t token_stride(const Tensor& x);

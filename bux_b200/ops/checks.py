@@ -2,7 +2,7 @@
 and run-twice determinism.
 
 ``BUX_KERNEL_CHECKS=1`` (or `enable()`) makes the wrappers in `bux_b200.ops.kernels`
-allocate each output inside a larger byte buffer whose head and tail are filled with a
+allocate each output (and each workspace) inside a larger byte buffer whose head and tail are filled with a
 pattern. `verify()` (call it after a synchronise; the GPU tests do after every test)
 reads the guards back and raises naming the op whose kernel wrote outside its output.
 A kernel that overruns therefore corrupts a guard of its own buffer instead of a
@@ -43,7 +43,7 @@ def enable(on: bool = True) -> None:
 
 
 def guarded_empty(shape, dtype, device, op: str, fill: Optional[float] = None) -> torch.Tensor:
-    """An uninitialised (or `fill`-ed) tensor for a kernel's output. With checks on it sits
+    """An uninitialised (or `fill`-ed) tensor for a kernel's output or workspace. With checks on it sits
     between two guard regions of `GUARD_BYTES` bytes each."""
     if not _on or torch.device(device).type != "cuda":
         if fill is None:

@@ -33,6 +33,19 @@ def _out(*shape, dtype, device, op: str, fill=None) -> torch.Tensor:
     return checks.guarded_empty(shape, dtype, device, op, fill)
 
 
+def _scratch(shape, dtype, device, op: str) -> Optional[torch.Tensor]:
+    """A workspace between guard regions with kernel checks on; else None (the op makes its own)."""
+    return _out(shape, dtype=dtype, device=device, op=op + " scratch") if checks.enabled() else None
+
+
+def _split_scratch(kind: int, m: int, n: int, k: int, bn: int, out_kind: int, sms: int, device, op: str) -> Optional[torch.Tensor]:
+    """The partial sums of a product whose contraction the op will split."""
+    if not checks.enabled() or bn or out_kind not in (OUT_BF16, OUT_F32):
+        return None
+    splits = ops().gemm_plan(kind, m, n, k, sms)[1]
+    return _scratch((splits, m, n), torch.float32, device, op) if splits > 1 else None
+
+
 def _count(n: int = 1) -> None:
     global _launches
     _launches += n
@@ -92,8 +105,10 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: boo
     if out is None:
         out = _out(m, n, dtype=out_dtype, device=a.device, op="gemm_bf16")
     kind = OUT_BF16 if out.dtype == torch.bfloat16 else (OUT_F32_ACC if accumulate else OUT_F32)
+    scratch = (_split_scratch(KIND_BF16, m, n, k, bn, kind, sms, a.device, "gemm_bf16")
+               if wait_flags is None and not m_rotate else None)
     ops().gemm(a, b, out, None, None, None, status_word(a.device), KIND_BF16, MODE_DENSE, m, n, k, k, 1,
-               a_mn, b_mn, kind, bn, sms, wait_flags, wait_epoch, wait_rows, m_rotate, wait_on_k, wait_on_n)
+               a_mn, b_mn, kind, bn, sms, wait_flags, wait_epoch, wait_rows, m_rotate, wait_on_k, wait_on_n, scratch)
     _count()
     return out
 
@@ -131,7 +146,8 @@ def gemm_mxfp8(aq, asf, bq, bsf, m: int, n: int, k: int, *, out=None, out_dtype=
         out = _out(m, n, dtype=out_dtype, device=aq.device, op="gemm_mxfp8")
     kind = OUT_BF16 if out.dtype == torch.bfloat16 else (OUT_F32_ACC if accumulate else OUT_F32)
     ops().gemm(aq.view(torch.uint8), bq.view(torch.uint8), out, asf, bsf, None, status_word(aq.device),
-               KIND_MXFP8, MODE_DENSE, m, n, k, k, 1, False, False, kind, bn, sms)
+               KIND_MXFP8, MODE_DENSE, m, n, k, k, 1, False, False, kind, bn, sms,
+               scratch=_split_scratch(KIND_MXFP8, m, n, k, bn, kind, sms, aq.device, "gemm_mxfp8"))
     _count()
     return out
 
@@ -286,7 +302,11 @@ def rmsnorm_bwd(x, w, dy, rstd, need_dw: bool = True):
     dx = _out(x.shape, dtype=x.dtype, device=x.device, op="rmsnorm_bwd dx")
     dw = (_out(x.shape[-1], dtype=torch.float32, device=x.device, op="rmsnorm_bwd dw")
           if need_dw and w is not None else None)
-    ops().rmsnorm_bwd(x, w, dy, rstd, dx, dw)
+    scratch = None
+    if dw is not None and checks.enabled():
+        parts = ops().rmsnorm_bwd_partials(x.numel() // x.shape[-1], x.shape[-1])
+        scratch = _scratch((parts, x.shape[-1]), torch.float32, x.device, "rmsnorm_bwd") if parts else None
+    ops().rmsnorm_bwd(x, w, dy, rstd, dx, dw, scratch)
     _count()
     return dx, dw
 
@@ -397,7 +417,9 @@ def sort_picks(experts: torch.Tensor, num_experts: int, align: int, rows: int, w
     pos = _out(experts.shape, dtype=torch.int32, device=dev, op="sort_picks pos")
     offsets = _out(num_experts + 1, dtype=torch.int32, device=dev, op="sort_picks offsets")
     w_row = _out(rows, dtype=torch.float32, device=dev, op="sort_picks w_row") if weights is not None else None
-    ops().sort_picks(experts, weights, row_index, pos, offsets, w_row, status_word(dev), align)
+    scratch = (_scratch((ops().pick_blocks(experts.numel()) + 1) * num_experts, torch.int32, dev, "sort_picks")
+               if checks.enabled() else None)
+    ops().sort_picks(experts, weights, row_index, pos, offsets, w_row, status_word(dev), align, scratch)
     _count(3)
     return row_index, pos, offsets, w_row
 

@@ -55,6 +55,36 @@ def test_guard_regions_hold_after_every_kernel_family(guarded):
     checks.verify()
 
 
+def test_workspaces_sit_between_guards_too(guarded):
+    """What an op would allocate for itself: the partial sums of a split product and of the gain's
+    gradient, the counts of the sort. Same results as without checks."""
+    from bux_b200.ops import kernels as K
+
+    dev = guarded
+    torch.manual_seed(3)
+    a, b = torch.randn(33, 4096, device=dev).bfloat16(), torch.randn(264, 4096, device=dev).bfloat16()
+    xq = K.quant_mxfp8(torch.randn(33, 8192, device=dev).bfloat16())
+    wq = K.quant_mxfp8(torch.randn(384, 8192, device=dev).bfloat16())
+    x, dy, w = torch.randn(301, 1032, device=dev).bfloat16(), torch.randn(301, 1032, device=dev).bfloat16(), torch.randn(1032, device=dev)
+    _, rstd = K.rmsnorm_fwd(x, w, 1e-6)
+    picks, wts = torch.randint(0, 7, (1500, 3), device=dev), torch.rand(1500, 3, device=dev)
+
+    def run():
+        return [K.gemm_bf16(a, b), K.gemm_mxfp8(xq[0], xq[1], wq[0], wq[1], 33, 384, 8192), *K.rmsnorm_bwd(x, w, dy, rstd),
+                *K.sort_picks(picks, 7, 16, 4608, wts)]
+
+    names = {"gemm_bf16 scratch", "gemm_mxfp8 scratch", "rmsnorm_bwd scratch", "sort_picks scratch"}
+    got = run()
+    torch.cuda.synchronize()
+    assert names <= {op for op, _, _ in checks._live}
+    checks.verify()
+    checks.enable(False)
+    assert all(torch.equal(p, q) for p, q in zip(got, run()))
+    checks.enable(True)
+    with pytest.raises(RuntimeError, match="scratch"):
+        K.ops().rmsnorm_bwd(x, w, dy, rstd, torch.empty_like(x), torch.empty_like(w), torch.empty(1, 1032, device=dev))
+
+
 def test_verify_names_the_op_whose_guard_was_overwritten(guarded):
     """A write past an output's end lands in its guard and is reported with the op's name.
     (The stray write is made by a host-side copy through a longer view, not by a kernel.)"""
