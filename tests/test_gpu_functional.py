@@ -301,8 +301,7 @@ def test_native_autograd_functions_match_the_python_ones(cuda, frozen, monkeypat
 
 
 def test_native_autograd_functions_refuse_and_recompute(cuda):
-    """Forward-mode differentiation stays refused; a checkpointed call recomputes; gradients of
-    gradients are not made up."""
+    """Forward-mode differentiation stays refused; a checkpointed call recomputes."""
     from torch.utils.checkpoint import checkpoint
 
     from bux_b200 import ops
@@ -319,8 +318,6 @@ def test_native_autograd_functions_refuse_and_recompute(cuda):
         else:
             again = torch.autograd.grad(y.sum(), [x, w])
         assert all(torch.equal(a, b) for a, b in zip(plain, again))
-    dx, = torch.autograd.grad(ops.rmsnorm(x, w).sum(), [x], create_graph=True)
-    assert not dx.requires_grad or dx.grad_fn is not None
     with pytest.raises((NotImplementedError, RuntimeError)):
         with torch.autograd.forward_ad.dual_level():
             ops.rmsnorm(torch.autograd.forward_ad.make_dual(x.detach(), torch.ones_like(x)), w)
@@ -432,3 +429,16 @@ def test_cross_entropy_head_takes_a_batch_of_gradients(cuda):
         one = torch.autograd.grad(ops.cross_entropy_head(x, w, tgt)[0], [x, w], s)
         for a, b in zip(many, one):
             assert a[i].dtype == b.dtype and torch.equal(a[i], b)
+
+
+@pytest.mark.parametrize("constant", [True, False])
+def test_gradients_of_native_functions_have_no_gradients(cuda, constant):
+    """The backward kernels are not differentiable: under create_graph the gradients do not pretend to
+    be, whether the incoming gradient depends on the inputs or not, and asking for theirs raises."""
+    for name, (inputs, fn) in _layer_calls(cuda).items():
+        xs = [x.detach().clone().requires_grad_() for x in inputs]
+        y = fn(*xs)
+        dx, = torch.autograd.grad(y, xs[:1], torch.ones_like(y) if constant else 2 * y, create_graph=True)
+        assert not dx.requires_grad, name
+        with pytest.raises(RuntimeError, match="does not require grad"):
+            torch.autograd.grad(dx.float().sum(), xs[:1])
