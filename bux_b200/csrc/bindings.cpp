@@ -317,6 +317,13 @@ void sort_picks(const Tensor& experts, const c10::optional<Tensor>& weights, Ten
                   row_index.data_ptr<int>(), pos.data_ptr<int>(), offsets.data_ptr<int>(), w_row.has_value() ? w_row->data_ptr<float>() : nullptr,
                   rows, work.data_ptr<int>(), status_ptr(status), stream_of(experts));
 }
+void pick_values(const Tensor& v, const Tensor& pos, Tensor& out) {
+  check_cuda(v, "v"); check_cuda(pos, "pos"); check_cuda(out, "out");
+  TORCH_CHECK(v.scalar_type() == at::kFloat && pos.scalar_type() == at::kInt && out.scalar_type() == at::kFloat && out.numel() == pos.numel(),
+              "pick_values: fp32 values, int32 rows, an fp32 output per row");
+  c10::cuda::CUDAGuard guard(v.device());
+  bux::pick_values(v.data_ptr<float>(), pos.data_ptr<int>(), out.data_ptr<float>(), pos.numel(), stream_of(v));
+}
 void gather_rows(const Tensor& x, const Tensor& index, Tensor& out) {
   check_cuda(x, "x"); check_cuda(out, "out");
   c10::cuda::CUDAGuard guard(x.device());
@@ -611,6 +618,7 @@ TORCH_LIBRARY(bux_b200, m) {
   m.def("sumsq(Tensor g, Tensor(a!) out) -> ()", &sumsq);
   m.def("topk_rows(Tensor scores, Tensor(a!) idx) -> ()", &topk_rows);
   m.def("sort_picks(Tensor experts, Tensor? weights, Tensor(a!) row_index, Tensor(b!) pos, Tensor(c!) offsets, Tensor(d!)? w_row, Tensor(e!)? status, int align, Tensor(f!)? scratch=None) -> ()", &sort_picks);
+  m.def("pick_values(Tensor v, Tensor pos, Tensor(a!) out) -> ()", &pick_values);
   m.def("gather_rows(Tensor x, Tensor index, Tensor(a!) out) -> ()", &gather_rows);
   m.def("combine_bwd(Tensor? y, Tensor dout, Tensor pos, Tensor? w, Tensor(a!)? dy, Tensor(b!)? dw) -> ()", &combine_bwd);
   m.def("combine_rows(Tensor y, Tensor pos, Tensor? w, Tensor(a!) out) -> ()", &combine_rows);

@@ -1483,6 +1483,13 @@ __global__ void gather_rows_kernel(const __nv_bfloat16* __restrict__ x, const in
     reinterpret_cast<uint4*>(out + r * d)[c] = v;
   }
 }
+// out[i] = v[pos[i]]; NaN for a pick of no expert (pos < 0).
+__global__ void pick_values_kernel(const float* __restrict__ v, const int* __restrict__ pos, float* __restrict__ out, long picks) {
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < picks; i += (long)gridDim.x * blockDim.x) {
+    const int r = pos[i];
+    out[i] = r < 0 ? __int_as_float(0x7fffffff) : v[r];
+  }
+}
 // out[t] = sum_k w[t,k] * y[pos[t,k]]  (pos < 0 = dropped pick; -2 = a pick of no expert, which
 // makes the row NaN); w may be null (= 1).
 __global__ void combine_rows_kernel(const __nv_bfloat16* __restrict__ y, const int* __restrict__ pos,
@@ -1727,6 +1734,9 @@ void sort_picks(const long long* experts, const float* weights, long n, int k, i
   pick_scan_kernel<<<1, 1024, 0, s>>>(work, blocks, E, align, totals, offsets);
   pick_place_kernel<<<blocks, PICK_THREADS, 8 * E * sizeof(int), s>>>(experts, weights, n, per_block, k, E, work, totals, offsets,
                                                                       row_index, pos, w_row, rows);
+}
+void pick_values(const float* v, const int* pos, float* out, long picks, cudaStream_t s) {
+  pick_values_kernel<<<grid_for(picks, 256), 256, 0, s>>>(v, pos, out, picks);
 }
 void gather_rows(const void* x, const int* index, void* out, long rows, int d, cudaStream_t s) {
   gather_rows_kernel<<<grid_for(rows * (d / 8), 256), 256, 0, s>>>((const __nv_bfloat16*)x, index, (__nv_bfloat16*)out, rows, d);

@@ -50,6 +50,8 @@ struct Status;
 int pick_blocks(long n);
 void sort_picks(const long long* experts, const float* weights, long n, int k, int E, int align, int* row_index, int* pos,
                 int* offsets, float* w_row, long rows, int* work, Status* st, cudaStream_t s);
+// out[i] = v[pos[i]], NaN where pos[i] < 0
+void pick_values(const float* v, const int* pos, float* out, long picks, cudaStream_t s);
 void gather_rows(const void* x, const int* index, void* out, long rows, int d, cudaStream_t s);
 void combine_bwd(const void* y, const void* dout, const int* pos, const float* w, void* dy, float* dw, long picks, int k, int d, cudaStream_t s);
 // causal depthwise convolution over the tokens (conv_sm100.cu): forward (bwd = false: out = y, `in` = x) and

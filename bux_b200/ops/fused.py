@@ -248,9 +248,8 @@ class _SortedExperts(torch.autograd.Function):
             # dh, and per row <da', glu(h)> = the gradient of that row's router weight
             dh, drs = K.glu_bwd(h, da, act, w_row, limit, up_offset)
             del da, h
-            # a pick of no expert has no row (its pos is negative): its weight's gradient is NaN, like its output
-            at = pos.long()
-            dwts[c * tc:(c + 1) * tc] = drs[at.clamp_min(0)].masked_fill_(at < 0, float("nan"))
+            # a pick of no expert has no row: its weight's gradient is NaN, like its token's output
+            K.pick_values_into(drs, pos, dwts[c * tc:(c + 1) * tc])
             if mx:
                 hq, hsf, htq, htsf = K.quant_mxfp8(dh, rowwise=True, colwise=True)
                 del dh

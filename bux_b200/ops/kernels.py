@@ -424,6 +424,12 @@ def sort_picks(experts: torch.Tensor, num_experts: int, align: int, rows: int, w
     return row_index, pos, offsets, w_row
 
 
+def pick_values_into(v, pos, out) -> None:
+    """out [t, k] = v[pos] of fp32 v [rows]; NaN for a pick of no expert (a negative pos, see `sort_picks`)."""
+    ops().pick_values(v, pos, out)
+    _count()
+
+
 def gather_rows(x, index, rows: int):
     out = _out(rows, x.shape[-1], dtype=x.dtype, device=x.device, op="gather_rows")
     ops().gather_rows(x, index, out)
