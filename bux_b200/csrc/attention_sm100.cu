@@ -24,7 +24,7 @@
 // SM). What shortened it, 8 x 4096 tokens, 32/4 heads of 128 (776 TFLOP/s at first): P in tensor memory
 // and two warps per scheduler and tile instead of one (888), P handed over in two parts so that the
 // tensor core starts on the first while the second is worked on, the maximum in a pass of its own
-// before them (1014). A third of the ex2 as polynomials on the FMA pipes was no gain (996): issue slots
+// before them (1004). A third of the ex2 as polynomials on the FMA pipes was no gain (996): issue slots
 // and tensor-memory latency, not that unit, fill the rest.
 //
 // Reference counterparts: cuDNN SDPA and FlashAttention-4 behind parallel/flash.py:573-678

@@ -35,7 +35,7 @@ struct AttnArgs {
 // walks the tiles of all heads with the longest walks first (tile 0 of every head, then tile 1, ...):
 // the short ones fill the gaps at the end. With the tiles of one head after another, long
 // walks of the last heads started late: the SMs had work 61 % of the backward's time (2 x 4096
-// tokens, 4 key heads, 256 blocks, forward + backward: 1796 us, now 1430) and 86 % of the forward's.
+// tokens, 4 key heads, 256 blocks, forward + backward: 1796 us, then 1409) and 86 % of the forward's.
 // Heads go 64 at a time, so that the keys in use stay within L2 however large the batch is. Where all
 // walks have about one length (no causal mask, or a window under half the row) the tiles of a head
 // stay together, since neighbours read the same keys.

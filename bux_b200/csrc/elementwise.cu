@@ -661,8 +661,7 @@ glu_bwd_rows_kernel(const __nv_bfloat16* __restrict__ h, const __nv_bfloat16* __
 
 // ---------------------------------------------------------------- MXFP8 quantiser
 // Tile: 128 rows x 128 columns per block of 256 threads, staged once in shared memory as
-// bf16 (row pitch 272 bytes: 16-byte accesses of 8 consecutive rows hit 8 different bank
-// groups). Each tile fills exactly one 512-byte scale tile of the row-wise output and one
+// bf16 (see qtile_at for its layout). Each tile fills exactly one 512-byte scale tile of the row-wise output and one
 // of the transposed output, written as whole tiles (padding scales included), and every
 // byte of both quantised outputs inside the padded extents, so the caller allocates
 // without clearing. Optional row gather (`row_index[r]` = source row of output row r,

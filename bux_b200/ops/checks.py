@@ -10,9 +10,10 @@ neighbour's data, and is named, which is what an address sanitizer would give, f
 writes that matter here (contiguous outputs of hand-written kernels).
 
 `same_twice(fn)` runs a function twice from the same inputs and reports the outputs that
-are not bitwise equal: the kernels here use no atomics on their outputs except where the
-docstring says so (dq's reduce-add, the RMSNorm weight gradient, the router-scale
-gradient), so anything else that differs between two runs is a race.
+are not bitwise equal: the kernels here use no atomics on their outputs except for dq's
+reduce-add, the gradients of the attention sinks and of the QK-norm gain, those of the RMSNorm
+gain for rows under 512 or over 8192 columns, the causal convolution's weight gradient and the
+sum of squares, so anything else that differs between two runs is a race.
 
 The reference has neither (it has no native code); its closest tool is XLA's
 deterministic-ops flag (``docs/parallelism/attention.md:322-323`` there).
