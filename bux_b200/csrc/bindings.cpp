@@ -90,7 +90,7 @@ void gemm(const Tensor& a, const Tensor& b, Tensor& c, const c10::optional<Tenso
   if (g.bn == 0) {   // the tile width and a split of the contraction are chosen here
     const bool may_split = g.mode == bux::MODE_DENSE && !wait_flags.has_value() && g.m_rotate == 0 &&
                            (out_kind == bux::OUT_BF16 || out_kind == bux::OUT_F32);
-    const bux::GemmPlan plan = bux::gemm_plan(g.kind, M, N, K, g.sms, may_split);
+    const bux::GemmPlan plan = bux::gemm_plan(g.kind, M, N, K, g.sms, may_split, g.a_mn);
     g.bn = plan.bn;
     if (plan.splits > 1) {
       partial = scratch_f32(scratch, {plan.splits, M, N}, c);
@@ -101,8 +101,8 @@ void gemm(const Tensor& a, const Tensor& b, Tensor& c, const c10::optional<Tenso
   TORCH_CHECK(err == nullptr, "bux gemm: ", err);
 }
 
-std::vector<int64_t> gemm_plan(int64_t kind, int64_t M, int64_t N, int64_t K, int64_t sms) {
-  const bux::GemmPlan plan = bux::gemm_plan((int)kind, M, N, K, (int)sms, true);
+std::vector<int64_t> gemm_plan(int64_t kind, int64_t M, int64_t N, int64_t K, int64_t sms, bool a_mn) {
+  const bux::GemmPlan plan = bux::gemm_plan((int)kind, M, N, K, (int)sms, true, a_mn);
   return {plan.bn, plan.splits, sms <= 0 && kind == bux::KIND_BF16 && plan.bn == 256 && plan.splits == 1 && bux::gemm_pairs(M, N, K)};
 }
 
@@ -608,7 +608,7 @@ TORCH_LIBRARY(bux_b200, m) {
   m.def("quant_mxfp8(Tensor x, Tensor? row_index, Tensor? row_scale, Tensor? q_row, Tensor? sf_row, Tensor? q_col, Tensor? sf_col, int rows, int cols, int ld_col, int batch, int x_batch_stride) -> ()", &quant_mxfp8);
   m.def("quant_mxfp8_glu(Tensor h, Tensor? dout, Tensor? row_scale, Tensor? q_row, Tensor? sf_row, Tensor? q_col, Tensor? sf_col, int ld_col, int kind, float limit, float up_offset) -> ()", &quant_mxfp8_glu);
   m.def("quant_nvfp4(Tensor x, Tensor tensor_scale, Tensor(a!) packed, Tensor(b!) scales) -> ()", &quant_nvfp4);
-  m.def("gemm_plan(int kind, int M, int N, int K, int sms=0) -> int[]", &gemm_plan);
+  m.def("gemm_plan(int kind, int M, int N, int K, int sms=0, bool a_mn=False) -> int[]", &gemm_plan);
   m.def("rmsnorm_bwd_partials(int rows, int d) -> int", [](int64_t rows, int64_t d) { return (int64_t)bux::rmsnorm_bwd_partials(rows, (int)d); });
   m.def("pick_blocks(int n) -> int", [](int64_t n) { return (int64_t)bux::pick_blocks(n); });
   m.def("token_stride(Tensor x) -> int", &token_stride);

@@ -724,7 +724,9 @@ __global__ void __launch_bounds__(256) sum_splits_kernel(const float* __restrict
 
 // One wave of 256-wide tiles costs 1, of 128-wide ones 0.62 (more operand traffic per product: 8192^3
 // 0.54, 32768 x 5120 x 2048 0.62, 16384 x 14336 x 4096 0.65 of the wide tile's time), so the narrow tile is
-// taken where it saves enough of a last wave. Where even its tiles leave half of the SMs idle, the
+// taken where it saves enough of a last wave. (0.69 where A's stored rows start off 128-byte lines: narrow
+// tiles read it twice as often; 3000 x 2048 x 18952 takes 254 us in three waves of them, 236 in two wide ones,
+// 200 on pairs.) Where even its tiles leave half of the SMs idle, the
 // contraction is cut as well, in ranges of at least four steps (the last may be shorter, none is
 // empty): a small product is a stream of its operands, and what bounds it is how many SMs read.
 // 16 x 6144 x 4096 (48 narrow tiles): 23.4 us with 24 wide tiles (29 with cold operands), 14.5 in 3 ranges
@@ -732,12 +734,13 @@ __global__ void __launch_bounds__(256) sum_splits_kernel(const float* __restrict
 // takes 0.2 us) and one for every 300000 values: the ranges have to save more. (Over 777 small products of
 // both kinds the faster of the two ways is missed by 0.3 %; always split 12 % slower, never 10 %. 128 x 2048 x
 // 512 in bf16 15.2 us split and 11.1 not, 300 x 1152 x 2048 in MXFP8 19.2 and 12.6, 16 x 4096 x 6144 19.5 and 21.5.)
-GemmPlan gemm_plan(int kind, long M, long N, long K, int sms, bool may_split) {
+GemmPlan gemm_plan(int kind, long M, long N, long K, int sms, bool may_split, bool a_mn) {
   if (sms <= 0) sms = GEMM_SMS;
   const long mt = (M + BM - 1) / BM, wide = mt * ((N + 255) / 256), narrow = mt * ((N + 127) / 128);
   const bool wide_fits = kind == KIND_BF16 || N % 256 == 0;
+  const double narrow_cost = kind == KIND_BF16 && (a_mn ? M : K) % 64 != 0 ? 0.69 : 0.62;
   GemmPlan plan{256, 1};
-  if (!wide_fits || (narrow + sms - 1) / sms * 0.62 < (double)((wide + sms - 1) / sms)) plan.bn = 128;
+  if (!wide_fits || (narrow + sms - 1) / sms * narrow_cost < (double)((wide + sms - 1) / sms)) plan.bn = 128;
   const long steps = (K + (kind == KIND_BF16 ? 63 : 127)) / (kind == KIND_BF16 ? 64 : 128);
   if (may_split && plan.bn == 128 && narrow > 0 && narrow * 2 <= sms && steps >= 8) {
     const long most = sms / narrow < steps / 4 ? sms / narrow : steps / 4, per = (steps + most - 1) / most;

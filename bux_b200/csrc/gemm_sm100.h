@@ -64,7 +64,7 @@ constexpr int GEMM_SMS = 148;   // SMs of the chip: a launch's blocks, and twice
 bool gemm_pairs(long M, long N, long K);
 // Tile width and number of contraction ranges for a dense product, from how full the SMs get.
 struct GemmPlan { int bn, splits; };
-GemmPlan gemm_plan(int kind, long M, long N, long K, int sms, bool may_split);
+GemmPlan gemm_plan(int kind, long M, long N, long K, int sms, bool may_split, bool a_mn);
 
 // Returns nullptr on success, else a static message.
 const char* gemm_launch(const GemmArgs& args, cudaStream_t stream);

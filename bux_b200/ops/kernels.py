@@ -38,11 +38,12 @@ def _scratch(shape, dtype, device, op: str) -> Optional[torch.Tensor]:
     return _out(shape, dtype=dtype, device=device, op=op + " scratch") if checks.enabled() else None
 
 
-def _split_scratch(kind: int, m: int, n: int, k: int, bn: int, out_kind: int, sms: int, device, op: str) -> Optional[torch.Tensor]:
+def _split_scratch(kind: int, m: int, n: int, k: int, a_mn: bool, bn: int, out_kind: int, sms: int, device,
+                   op: str) -> Optional[torch.Tensor]:
     """The partial sums of a product whose contraction the op will split."""
     if not checks.enabled() or bn or out_kind not in (OUT_BF16, OUT_F32):
         return None
-    splits = ops().gemm_plan(kind, m, n, k, sms)[1]
+    splits = ops().gemm_plan(kind, m, n, k, sms, a_mn)[1]
     return _scratch((splits, m, n), torch.float32, device, op) if splits > 1 else None
 
 
@@ -105,7 +106,7 @@ def gemm_bf16(a: torch.Tensor, b: torch.Tensor, *, a_mn: bool = False, b_mn: boo
     if out is None:
         out = _out(m, n, dtype=out_dtype, device=a.device, op="gemm_bf16")
     kind = OUT_BF16 if out.dtype == torch.bfloat16 else (OUT_F32_ACC if accumulate else OUT_F32)
-    scratch = (_split_scratch(KIND_BF16, m, n, k, bn, kind, sms, a.device, "gemm_bf16")
+    scratch = (_split_scratch(KIND_BF16, m, n, k, a_mn, bn, kind, sms, a.device, "gemm_bf16")
                if wait_flags is None and not m_rotate else None)
     ops().gemm(a, b, out, None, None, None, status_word(a.device), KIND_BF16, MODE_DENSE, m, n, k, k, 1,
                a_mn, b_mn, kind, bn, sms, wait_flags, wait_epoch, wait_rows, m_rotate, wait_on_k, wait_on_n, scratch)
@@ -147,7 +148,7 @@ def gemm_mxfp8(aq, asf, bq, bsf, m: int, n: int, k: int, *, out=None, out_dtype=
     kind = OUT_BF16 if out.dtype == torch.bfloat16 else (OUT_F32_ACC if accumulate else OUT_F32)
     ops().gemm(aq.view(torch.uint8), bq.view(torch.uint8), out, asf, bsf, None, status_word(aq.device),
                KIND_MXFP8, MODE_DENSE, m, n, k, k, 1, False, False, kind, bn, sms,
-               scratch=_split_scratch(KIND_MXFP8, m, n, k, bn, kind, sms, aq.device, "gemm_mxfp8"))
+               scratch=_split_scratch(KIND_MXFP8, m, n, k, False, bn, kind, sms, aq.device, "gemm_mxfp8"))
     _count()
     return out
 

@@ -34,6 +34,14 @@ def test_pairs_of_sms_take_what_fills_them(m, n, k, pairs):
     assert not K.ops().gemm_plan(K.KIND_MXFP8, m, n, k)[2]
 
 
+@pytest.mark.parametrize("m,n,k,a_mn,width", [(3000, 2048, 18952, False, 256), (3000, 2048, 18944, False, 128),
+                                              (3000, 2048, 18952, True, 256), (3008, 2048, 18952, True, 128),
+                                              (776, 2048, 5128, False, 128)])
+def test_narrow_tiles_and_rows_off_whole_lines(m, n, k, a_mn, width):
+    """Three narrow waves against two wide ones, unless A's rows start off 128-byte lines; one against one."""
+    assert K.ops().gemm_plan(K.KIND_BF16, m, n, k, 0, a_mn)[0] == width
+
+
 @pytest.mark.parametrize("kind,m,n,k,splits", [
     (K.KIND_BF16, 16, 6144, 4096, 3), (K.KIND_BF16, 1, 2048, 2880, 9), (K.KIND_MXFP8, 16, 4096, 6144, 4),
     (K.KIND_BF16, 128, 2048, 512, 1), (K.KIND_BF16, 16, 8192, 1024, 1), (K.KIND_MXFP8, 300, 1152, 2048, 1)])
